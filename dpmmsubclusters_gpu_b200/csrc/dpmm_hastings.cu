@@ -19,13 +19,13 @@ namespace dpmm {
 // one block per slot (3K): log marginal likelihood of each cluster / sub-cluster
 // sel (nullable): clusters whose slots use the second prior (k1, v1, ld1, prior1), the outlier layout
 template <int DP>
-__global__ void __launch_bounds__(RegChol<DP>::T) k_slot_lml(const double* __restrict__ stats, int stat_len, int D,
+__global__ void __launch_bounds__(BlockChol<DP>::T) k_slot_lml(const double* __restrict__ stats, int stat_len, int D,
                                                              int gauss, double k0, double v0, double ld0,
                                                              const double* __restrict__ prior, double k1, double v1,
                                                              double ld1, const double* __restrict__ prior1,
                                                              const uint8_t* __restrict__ sel, double* __restrict__ lml)
 {
-    __shared__ double sh[RegChol<DP>::SMEM];
+    extern __shared__ double sh[];
     if (sel && sel[blockIdx.x / 3]) {
         k0 = k1;
         v0 = v1;
@@ -35,9 +35,9 @@ __global__ void __launch_bounds__(RegChol<DP>::T) k_slot_lml(const double* __res
     const double* st = stats + (size_t)blockIdx.x * stat_len;
     double v;
     if (gauss)
-        v = niw_lml_reg<DP>(D, st[0], st + 1, st + 1 + D, nullptr, nullptr, k0, v0, prior, prior + D, ld0, sh);
+        v = niw_lml_block<DP>(D, st[0], st + 1, st + 1 + D, nullptr, nullptr, k0, v0, prior, prior + D, ld0, sh);
     else
-        v = mult_lml_block(D, st[0], st + 1, nullptr, prior, sh + 3 * DP);
+        v = mult_lml_block(D, st[0], st + 1, nullptr, prior, sh + BlockChol<DP>::RED);
     if (threadIdx.x == 0) lml[blockIdx.x] = v;
 }
 
@@ -52,7 +52,7 @@ __global__ void k_split_hr(const double* __restrict__ stats, int stat_len, const
 // one block per pair i < j: statistics aggregated (niw.cpp:140-148), posterior, lml, ratio
 // the merged cluster takes cluster i's prior (shared_actions.cpp:88-95): the second one where sel[i]
 template <int DP>
-__global__ void __launch_bounds__(RegChol<DP>::T) k_merge_hr(const double* __restrict__ stats, int stat_len, int D,
+__global__ void __launch_bounds__(BlockChol<DP>::T) k_merge_hr(const double* __restrict__ stats, int stat_len, int D,
                                                              int gauss, double k0, double v0, double ld0,
                                                              const double* __restrict__ prior, double k1, double v1,
                                                              double ld1, const double* __restrict__ prior1,
@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(RegChol<DP>::T) k_merge_hr(const double* __res
                                                              const double* __restrict__ lml, int K, double alpha,
                                                              double* __restrict__ hr)
 {
-    __shared__ double sh[RegChol<DP>::SMEM];
+    extern __shared__ double sh[];
     // unrank pair b -> (i, j), i < j, row-major over the strict upper triangle
     long long b = blockIdx.x;
     int i = 0;
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(RegChol<DP>::T) k_merge_hr(const double* __res
         ld0 = ld1;
         prior = prior1;
     }
-    const double v = merge_log_hr_reg<DP>(stats, stat_len, D, gauss, k0, v0, ld0, prior, lml, i, j, alpha, sh);
+    const double v = merge_log_hr_block<DP>(stats, stat_len, D, gauss, k0, v0, ld0, prior, lml, i, j, alpha, sh);
     if (threadIdx.x == 0) hr[(size_t)i * K + j] = v;
 }
 
@@ -84,7 +84,8 @@ static dpmm_status launch_slot_lml(dpmm_ctx* c, int K)
 {
     const int gauss = c->prior == DPMM_PRIOR_GAUSSIAN;
     const bool out = c->outlier_layout != 0;
-    DPMM_WITH_DP(chol_dp(c), (k_slot_lml<DP><<<3 * K, RegChol<DP>::T, 0, c->stream>>>(
+    DPMM_WITH_DP(chol_dp(c), DPMM_TRY(allow_smem(k_slot_lml<DP>, BlockChol<DP>::bytes));
+                 (k_slot_lml<DP><<<3 * K, BlockChol<DP>::T, BlockChol<DP>::bytes, c->stream>>>(
                                  c->d_stats, c->stat_len, c->D, gauss, c->prior_k, c->prior_v, c->prior_logdet,
                                  c->d_prior, c->prior2_k, c->prior2_v, c->prior2_logdet,
                                  out ? c->d_prior2 : c->d_prior, out ? c->d_prior_sel : nullptr, c->d_lml)));
@@ -123,7 +124,8 @@ dpmm_status launch_merge_hastings(dpmm_ctx* c, int K, double alpha)
     if (pairs == 0) return DPMM_OK;
     const int gauss = c->prior == DPMM_PRIOR_GAUSSIAN;
     const bool out = c->outlier_layout != 0;
-    DPMM_WITH_DP(chol_dp(c), (k_merge_hr<DP><<<(unsigned)pairs, RegChol<DP>::T, 0, c->stream>>>(
+    DPMM_WITH_DP(chol_dp(c), DPMM_TRY(allow_smem(k_merge_hr<DP>, BlockChol<DP>::bytes));
+                 (k_merge_hr<DP><<<(unsigned)pairs, BlockChol<DP>::T, BlockChol<DP>::bytes, c->stream>>>(
                                  c->d_stats, c->stat_len, c->D, gauss, c->prior_k, c->prior_v, c->prior_logdet,
                                  c->d_prior, c->prior2_k, c->prior2_v, c->prior2_logdet, out ? c->d_prior2 : c->d_prior,
                                  out ? c->d_prior_sel : nullptr, c->d_lml, K, alpha, c->d_merge_hr)));
@@ -147,48 +149,48 @@ static __device__ __align__(256) double g_merge_scratch[1 + kStaticMaxClusters];
 
 // scratch[0] = log det psi0 (NIW prior)
 template <int DP>
-__global__ void __launch_bounds__(RegChol<DP>::T) k_static_prior_logdet(const double* __restrict__ prior, int D,
+__global__ void __launch_bounds__(BlockChol<DP>::T) k_static_prior_logdet(const double* __restrict__ prior, int D,
                                                                          double* __restrict__ scratch)
 {
-    using RC = RegChol<DP>;
-    __shared__ double sh[RC::SMEM];
-    const int i = threadIdx.x % DP, c = threadIdx.x / DP;
-    double a[RC::EP];
-#pragma unroll
-    for (int q = 0; q < RC::EP; ++q) {
-        const int k = c + q * RC::C;
-        a[q] = (c < RC::C && i < D && k <= i) ? prior[D + (size_t)i * D + k] : 0.0;   // psi0(k, i), k <= i
+    using BC = BlockChol<DP>;
+    extern __shared__ double sh[];
+    for (int e = threadIdx.x; e < D * D; e += blockDim.x) {
+        const int i = e / D, k = e % D;
+        if (k <= i) sh[i * BC::LD + k] = prior[D + (size_t)i * D + k];   // psi0(k, i), k <= i
     }
-    const double ld = reg_chol_logdet<DP>(a, D, sh, nullptr);
+    __syncthreads();
+    if (threadIdx.x < 32) warp_ldl<DP>(sh, D, sh + BC::PIV);
+    __syncthreads();
+    const double ld = block_log_pivots<DP>(D, sh + BC::PIV, sh + BC::RED);
     if (threadIdx.x == 0) scratch[0] = ld;
 }
 
 // scratch[1 + k] = log marginal likelihood of cluster k (statistics slot 3k)
 template <int DP>
-__global__ void __launch_bounds__(RegChol<DP>::T) k_static_cluster_lml(const double* __restrict__ stats, int stat_len,
+__global__ void __launch_bounds__(BlockChol<DP>::T) k_static_cluster_lml(const double* __restrict__ stats, int stat_len,
                                                                         int D, int gauss, double k0, double v0,
                                                                         const double* __restrict__ prior,
                                                                         double* __restrict__ scratch)
 {
-    __shared__ double sh[RegChol<DP>::SMEM];
+    extern __shared__ double sh[];
     const double* st = stats + (size_t)(3 * blockIdx.x) * stat_len;
     double v;
     if (gauss)
-        v = niw_lml_reg<DP>(D, st[0], st + 1, st + 1 + D, nullptr, nullptr, k0, v0, prior, prior + D, scratch[0], sh);
+        v = niw_lml_block<DP>(D, st[0], st + 1, st + 1 + D, nullptr, nullptr, k0, v0, prior, prior + D, scratch[0], sh);
     else
-        v = mult_lml_block(D, st[0], st + 1, nullptr, prior, sh + 3 * DP);
+        v = mult_lml_block(D, st[0], st + 1, nullptr, prior, sh + BlockChol<DP>::RED);
     if (threadIdx.x == 0) scratch[1 + blockIdx.x] = v;
 }
 
 // one block per pair i < j, as k_merge_hr, with the per-cluster terms read from the scratch
 template <int DP>
-__global__ void __launch_bounds__(RegChol<DP>::T) k_static_merge_hr(const double* __restrict__ stats, int stat_len,
+__global__ void __launch_bounds__(BlockChol<DP>::T) k_static_merge_hr(const double* __restrict__ stats, int stat_len,
                                                                      int D, int gauss, double k0, double v0,
                                                                      const double* __restrict__ prior,
                                                                      const double* __restrict__ scratch, int K,
                                                                      double alpha, double* __restrict__ hr)
 {
-    __shared__ double sh[RegChol<DP>::SMEM];
+    extern __shared__ double sh[];
     long long b = blockIdx.x;
     int i = 0;
     long long rowlen = K - 1;
@@ -200,10 +202,10 @@ __global__ void __launch_bounds__(RegChol<DP>::T) k_static_merge_hr(const double
     if (ni == 0 || nj == 0) return;       // stays NaN
     double lij;
     if (gauss)
-        lij = niw_lml_reg<DP>(D, ni + nj, si + 1, si + 1 + D, sj + 1, sj + 1 + D, k0, v0, prior, prior + D, scratch[0],
+        lij = niw_lml_block<DP>(D, ni + nj, si + 1, si + 1 + D, sj + 1, sj + 1 + D, k0, v0, prior, prior + D, scratch[0],
                               sh);
     else
-        lij = mult_lml_block(D, ni + nj, si + 1, sj + 1, prior, sh + 3 * DP);
+        lij = mult_lml_block(D, ni + nj, si + 1, sj + 1, prior, sh + BlockChol<DP>::RED);
     if (threadIdx.x != 0) return;
     const double n = ni + nj;
     hr[(size_t)i * K + j] = -log(alpha) + lgamma(alpha) - 2 * lgamma(0.5 * alpha) + lgamma(n) - lgamma(n + alpha) +
@@ -298,15 +300,18 @@ extern "C" dpmm_status dpmm_merge_hastings_static(int32_t prior_type, int32_t D,
     const int dp = gauss ? padded_dim(D) : 4;
     DPMM_CUDA_TRY(cudaMemsetAsync(merge_log_hr, 0xff, sizeof(double) * (size_t)K * K, s));   // NaN
     if (gauss) {
-        DPMM_WITH_DP(dp, (k_static_prior_logdet<DP><<<1, RegChol<DP>::T, 0, s>>>(prior, D, scratch)));
+        DPMM_WITH_DP(dp, DPMM_TRY(allow_smem(k_static_prior_logdet<DP>, BlockChol<DP>::bytes));
+                 (k_static_prior_logdet<DP><<<1, BlockChol<DP>::T, BlockChol<DP>::bytes, s>>>(prior, D, scratch)));
         DPMM_LAUNCHED();
     }
-    DPMM_WITH_DP(dp, (k_static_cluster_lml<DP><<<K, RegChol<DP>::T, 0, s>>>(stats, stat_len, D, gauss ? 1 : 0, k0, v0,
+    DPMM_WITH_DP(dp, DPMM_TRY(allow_smem(k_static_cluster_lml<DP>, BlockChol<DP>::bytes));
+                 (k_static_cluster_lml<DP><<<K, BlockChol<DP>::T, BlockChol<DP>::bytes, s>>>(stats, stat_len, D, gauss ? 1 : 0, k0, v0,
                                                                             prior, scratch)));
     DPMM_LAUNCHED();
     const long long pairs = (long long)K * (K - 1) / 2;
     if (pairs > 0) {
-        DPMM_WITH_DP(dp, (k_static_merge_hr<DP><<<(unsigned)pairs, RegChol<DP>::T, 0, s>>>(
+        DPMM_WITH_DP(dp, DPMM_TRY(allow_smem(k_static_merge_hr<DP>, BlockChol<DP>::bytes));
+                 (k_static_merge_hr<DP><<<(unsigned)pairs, BlockChol<DP>::T, BlockChol<DP>::bytes, s>>>(
                              stats, stat_len, D, gauss ? 1 : 0, k0, v0, prior, scratch, K, alpha, merge_log_hr)));
         DPMM_LAUNCHED();
     }

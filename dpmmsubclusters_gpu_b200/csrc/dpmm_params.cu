@@ -92,8 +92,12 @@ __device__ double chi2_draw(double k, uint64_t seed, uint64_t draw, uint32_t s, 
 // (cluster 1, local_clusters_actions.cpp:348-351) keep their parameters: only their log marginal
 // likelihood and the cluster slot's weight term are refreshed (cbase[s] = -log det Sigma / 2 of the
 // slot's current parameters, written by every draw).
+// Bound: three chains one after the other, the factorisation (see BlockChol), the rows of the inverse (8 clocks
+// a term, 2016 terms at D = 64; A^T y = z runs beside it) and the products W = L^-T A.  The variates come from
+// the warps that do not factor, beside the factorisation.  Measured: 300 slots at D = 64 258 -> 85 us, 192 at
+// D = 50 186 -> 67 us, 60 at D = 32 85 -> 40 us.
 template <int DP>
-__global__ void __launch_bounds__(RegChol<DP>::T) k_draw_niw(const double* __restrict__ stats, int stat_len, int D,
+__global__ void __launch_bounds__(BlockChol<DP>::T) k_draw_niw(const double* __restrict__ stats, int stat_len, int D,
                                                               int Dp, double k0, double v0, double ld0,
                                                               const double* __restrict__ prior, double k1, double v1,
                                                               double ld1, const double* __restrict__ prior1,
@@ -106,13 +110,14 @@ __global__ void __launch_bounds__(RegChol<DP>::T) k_draw_niw(const double* __res
                                                               float* __restrict__ muv, double* __restrict__ lml,
                                                               int* __restrict__ err)
 {
-    __shared__ double sh[RegChol<DP>::SMEM];
-    __shared__ double mean[DP], yv[DP], zv[DP], uv[DP];
+    using BC = BlockChol<DP>;
+    constexpr int LD = BC::LD;
+    __shared__ double mean[DP], yv[DP], zv[DP], uv[DP], xd[DP];
     extern __shared__ double dyn[];
-    const int AL = D + 1;                  // leading dimension of A: column reads across lanes are conflict-free
-    double* Lm = dyn;                      // D*D: Cholesky factor of psi', later its inverse
-    double* Am = Lm + (size_t)D * D;       // D*AL: Bartlett factor (lower)
-    double* red = sh + 3 * DP;
+    constexpr int AL = DP + 1;             // leading dimension of A: column reads across lanes are conflict-free
+    double* sh = dyn;                      // the factorisation's memory: psi' -> L -> L^-1
+    double* Am = dyn + BC::SMEM;           // DP*AL: Bartlett factor (lower), column-major, zero above
+    double* red = sh + BC::RED;
     const int s = blockIdx.x, t = threadIdx.x;
     if (sel && sel[s / 3]) {   // the outlier prior
         k0 = k1;
@@ -123,76 +128,111 @@ __global__ void __launch_bounds__(RegChol<DP>::T) k_draw_niw(const double* __res
     const double* st = stats + (size_t)s * stat_len;
     const double n = st[0];
     const double kp = k0 + n, vp = v0 + n;
-    for (int e = t; e < D * D; e += blockDim.x) Lm[e] = 0.0;
-    __syncthreads();
+    const bool keep = s >= skip_lo && s < skip_hi;   // parameters kept (uniform over the block)
+    const uint32_t us = (uint32_t)s;
+    // the variates need no factor: the warps that do not factor make them meanwhile, the rejection loops of
+    // the diagonal first
+    auto variates = [&](int tt, int nt) {
+        if (keep) return;
+        for (int i = tt; i < D; i += nt) Am[i * AL + i] = sqrt(chi2_draw(vp - i, seed, draw, us, (uint32_t)(D * D + 256 * i)));
+        for (int i = nt - 1 - tt; i < D; i += nt)
+            zv[i] = normal_from(param_bits(seed, draw, (uint32_t)(D * D + 256 * D + i), us));
+        const int total = D / 2 * (D - 1) + (D & 1) * (D / 2);   // D (D - 1) / 2 below the diagonal
+        for (int e = tt; e < total; e += nt) {
+            int i, j;
+            strict_lower(D, e, i, j);
+            Am[j * AL + i] = normal_from(param_bits(seed, draw, (uint32_t)(j * D + i), us));
+        }
+    };
+    for (int e = t; e < DP * AL; e += blockDim.x) Am[e] = 0.0;   // (the barriers of the posterior order it)
     NiwExtras ex;
-    const double L = niw_lml_reg<DP>(D, n, st + 1, st + 1 + D, nullptr, nullptr, k0, v0, prior, prior + D, ld0, sh,
-                                     &ex, Lm, true);
-    if (s >= skip_lo && s < skip_hi) {   // parameters kept (uniform over the block)
+    const double L = niw_lml_block<DP>(D, n, st + 1, st + 1 + D, nullptr, nullptr, k0, v0, prior, prior + D, ld0, sh, &ex,
+                                       true, variates);
+    if (keep) {
         if (t == 0) {
             lml[s] = n > 0 ? L : 0.0;
             if (s % 3 == 0) cv[s] = (float)(cbase[s] + logw[s / 3]);
         }
         return;
     }
-    const double* mp = sh + 2 * DP;        // posterior mean, left by niw_lml_reg
-    const uint32_t us = (uint32_t)s;
-    for (int e = t; e < D * D; e += blockDim.x) {
-        const int i = e % D, j = e / D;
-        double v = 0.0;
-        if (i > j) v = normal_from(param_bits(seed, draw, (uint32_t)e, us));
-        else if (i == j) v = sqrt(chi2_draw(vp - i, seed, draw, us, (uint32_t)(D * D + 256 * i)));
-        Am[(size_t)j * AL + i] = v;
-    }
-    for (int i = t; i < D; i += blockDim.x) zv[i] = normal_from(param_bits(seed, draw, (uint32_t)(D * D + 256 * D + i), us));
-    __syncthreads();
-    // A^T y = z (A^T upper triangular), one warp, rows from the last
-    if (t < 32) {
+    const double* mp = sh + BC::MP;        // posterior mean, left by niw_lml_block
+    block_ldl_to_cholesky<DP>(sh, D, sh + BC::PIV, xd);
+    // the inverse of L (a row per thread of the first DP) and, by the last warp, A^T y = z (A^T upper
+    // triangular), rows from the last: two chains side by side
+    if (t < DP) rows_tri_inverse<DP>(sh, D, xd, t);
+    if (t >= (int)blockDim.x - 32) {
+        const int lane = t & 31;
         for (int i = D - 1; i >= 0; --i) {
             double p = 0;
-            for (int q = i + 1 + t; q < D; q += 32) p += Am[(size_t)i * AL + q] * yv[q];
+            for (int q = i + 1 + lane; q < D; q += 32) p += Am[i * AL + q] * yv[q];
             p = warp_sum_d(p);
-            if (t == 0) yv[i] = (zv[i] - p) / Am[(size_t)i * AL + i];
+            if (lane == 0) yv[i] = (zv[i] - p) / Am[i * AL + i];
             __syncwarp();
         }
     }
     __syncthreads();
+    auto Lf = [&](int i, int j) { return sh[j * LD + i]; };                           // L(i, j), j <= i
+    auto X = [&](int i, int j) { return i == j ? xd[i] : sh[i * LD + j]; };           // L^-1(i, j), j <= i
     // mu = m' + L_B y / sqrt(kappa'), L_B = sqrt(nu') L (the factor of nu' psi')
     const double sv = sqrt(vp), isk = 1.0 / sqrt(kp);
     for (int i = t; i < D; i += blockDim.x) {
         double acc = 0;
-        for (int q = 0; q <= i; ++q) acc += Lm[(size_t)q * D + i] * yv[q];
+        for (int q = 0; q <= i; ++q) acc += Lf(i, q) * yv[q];
         mean[i] = mp[i] + sv * acc * isk;
     }
     double la = 0;
-    for (int i = t; i < D; i += blockDim.x) la += log(Am[(size_t)i * AL + i]);
-    la = block_sum(la, red);               // (its barriers also order mean[] before the inverse)
+    for (int i = t; i < D; i += blockDim.x) la += log(Am[i * AL + i]);
+    la = block_sum(la, red);               // (its barriers also order mean[])
     const double logdet_sigma = D * log(vp) + ex.ld - 2.0 * la;
-    block_tri_inverse(Lm, D);              // Lm = L^-1 (lower)
     // u = L^-1 (mu - shift); b_j = sum_i W(i, j) (mu_i - shift_i) = (1/sqrt(nu')) sum_{k >= j} A(k, j) u_k
     for (int k = t; k < D; k += blockDim.x) {
         double acc = 0;
-        for (int i = 0; i <= k; ++i) acc += Lm[(size_t)i * D + k] * (mean[i] - shift[i]);
+        for (int i = 0; i <= k; ++i) acc += X(k, i) * (mean[i] - shift[i]);
         uv[k] = acc;
+    }
+    // L^-1 becomes plain lower triangular with zeros above, so that the products below need no case
+    __syncthreads();
+    for (int e = t; e < DP * DP; e += blockDim.x) {
+        const int i = e / DP, k = e % DP;
+        if (k >= i || i >= D) sh[i * LD + k] = i == k && i < D ? xd[i] : 0.0;
     }
     __syncthreads();
     const float isv = (float)(1.0 / sv);
     float* wt = Wt + (size_t)s * Dp * Dp;
-    // W(i, j) = (1/sqrt(nu')) sum_{k >= max(i, j)} L^-1(k, i) A(k, j); Wt[j][i] = W(i, j); lanes take j
-    for (int e = t; e < Dp * Dp; e += blockDim.x) {
-        const int i = e / Dp, j = e % Dp;
-        float w = 0.f;
-        if (i < D && j < D) {
-            double acc = 0;
-            for (int k = max(i, j); k < D; ++k) acc += Lm[(size_t)i * D + k] * Am[(size_t)j * AL + k];
-            w = (float)acc * isv;
+    // W(i, j) = (1/sqrt(nu')) sum_{k >= max(i, j)} L^-1(k, i) A(k, j); Wt[j][i] = W(i, j).  A thread takes 4 x TJ
+    // outputs: the terms below max(i, j) are products with a zero and leave the sum as it is
+    {
+        constexpr int TJ = DP >= 64 ? 8 : DP >= 32 ? 2 : 1, NI = DP / 4, NJ = DP / TJ;
+        for (int tile = t; tile < NI * NJ; tile += blockDim.x) {
+            const int i0 = tile % NI, j0 = TJ * (tile / NI);   // i = i0 + NI a, j = j0 + b
+            double acc[4][TJ];
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < TJ; ++b) acc[a][b] = 0.0;
+#pragma unroll 2
+            for (int k = max(i0, j0); k < D; ++k) {
+                double xv[4], av[TJ];
+#pragma unroll
+                for (int a = 0; a < 4; ++a) xv[a] = sh[k * LD + i0 + NI * a];
+#pragma unroll
+                for (int b = 0; b < TJ; ++b) av[b] = Am[(j0 + b) * AL + k];
+#pragma unroll
+                for (int a = 0; a < 4; ++a)
+#pragma unroll
+                    for (int b = 0; b < TJ; ++b) acc[a][b] += xv[a] * av[b];
+            }
+#pragma unroll
+            for (int b = 0; b < TJ; ++b)
+#pragma unroll
+                for (int a = 0; a < 4; ++a)
+                    wt[(size_t)(j0 + b) * DP + i0 + NI * a] = i0 + NI * a < D && j0 + b < D ? (float)acc[a][b] * isv : 0.f;
         }
-        wt[(size_t)j * Dp + i] = w;
     }
     for (int j = t; j < Dp; j += blockDim.x) {
         double b = 0;
         if (j < D)
-            for (int k = j; k < D; ++k) b += Am[(size_t)j * AL + k] * uv[k];
+            for (int k = j; k < D; ++k) b += Am[j * AL + k] * uv[k];
         bv[(size_t)s * Dp + j] = j < D ? (float)(b / sv) : 0.f;
         muv[(size_t)s * Dp + j] = j < D ? (float)(mean[j] - shift[j]) : 0.f;
     }
@@ -284,10 +324,10 @@ static dpmm_status launch_draw_niw(dpmm_ctx* c, int K, uint64_t seed, uint64_t d
     if constexpr (DP > 64) {
         return fail(DPMM_ERR_INVALID_ARG, "device draws need D <= 64");
     } else {
-        const size_t sm = sizeof(double) * ((size_t)c->D * c->D + (size_t)c->D * (c->D + 1));
+        constexpr size_t sm = sizeof(double) * (BlockChol<DP>::SMEM + (size_t)DP * (DP + 1));
         DPMM_TRY(allow_smem(k_draw_niw<DP>, sm));
         const bool out = c->outlier_layout != 0;
-        k_draw_niw<DP><<<3 * K, RegChol<DP>::T, sm, c->stream>>>(
+        k_draw_niw<DP><<<3 * K, BlockChol<DP>::T, sm, c->stream>>>(
             c->d_stats, c->stat_len, c->D, c->Dp, c->prior_k, c->prior_v, c->prior_logdet, c->d_prior, c->prior2_k,
             c->prior2_v, c->prior2_logdet, out ? c->d_prior2 : c->d_prior, out ? c->d_prior_sel : nullptr,
             out ? 3 : 0, out && K > 1 ? 6 : 0, c->d_cbase, c->d_gshift, c->d_logw, seed, draw, c->d_Wt, c->d_b, c->d_c, c->d_mu,

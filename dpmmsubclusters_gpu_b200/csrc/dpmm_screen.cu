@@ -146,17 +146,17 @@ __device__ void screen_assemble(float* __restrict__ f, bool merge, bool gauss, i
 // NIW: one block per slot (3K).  vec[s] = posterior mean m'[D] then diag(psi')[D].  Cluster slots also
 // get the exact log marginal likelihood, log det psi', tau and the inverse Cholesky factor of psi'.
 // psi0_identity: the prior scale is the identity and its mean zero (tau needs no prior matrix then).
-// Dynamic shared memory: D*D doubles (the Cholesky factor, then its inverse).
+// Dynamic shared memory: BlockChol<DP>::SMEM doubles.
 template <int DP>
-__global__ void __launch_bounds__(RegChol<DP>::T) k_screen_slots_niw(const double* __restrict__ stats, int stat_len,
+__global__ void __launch_bounds__(BlockChol<DP>::T) k_screen_slots_niw(const double* __restrict__ stats, int stat_len,
                                                                       int D, double k0, double v0, double ld0,
                                                                       const double* __restrict__ prior,
                                                                       int psi0_identity, double* __restrict__ rec,
                                                                       double* __restrict__ vec, float* __restrict__ linv)
 {
-    __shared__ double sh[RegChol<DP>::SMEM];
-    extern __shared__ double Lm[];
-    double* red = sh + 3 * DP;
+    using BC = BlockChol<DP>;
+    extern __shared__ double sh[];
+    double* red = sh + BlockChol<DP>::RED;
     const int s = blockIdx.x;
     const double* st = stats + (size_t)s * stat_len;
     const double n = st[0];
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(RegChol<DP>::T) k_screen_slots_niw(const doubl
     const double kp = k0 + n, vp = v0 + n;
     double h = 0, t = 0;
     for (int d = threadIdx.x; d < D; d += blockDim.x) {
-        // the expressions of niw_lml_reg for m'[d] and psi'(d, d)
+        // the expressions of niw_lml_block for m'[d] and psi'(d, d)
         const double m = (m0[d] * k0 + st[1 + d]) / kp;
         const size_t dd = (size_t)d * D + d;
         const double tm = v0 * psi0[dd] + k0 * m0[d] * m0[d];
@@ -181,32 +181,31 @@ __global__ void __launch_bounds__(RegChol<DP>::T) k_screen_slots_niw(const doubl
     double ld = 0, L = 0, tau = 0;
     if (s % 3 == 0 && n > 0) {
         NiwExtras ex;
-        L = niw_lml_reg<DP>(D, n, st + 1, st + 1 + D, nullptr, nullptr, k0, v0, m0, psi0, ld0, sh, &ex, Lm);
+        L = niw_lml_block<DP>(D, n, st + 1, st + 1 + D, nullptr, nullptr, k0, v0, m0, psi0, ld0, sh, &ex);
         ld = ex.ld;
         h = ex.hd;
         t = ex.tr;
-        for (int e = threadIdx.x; e < D * D; e += blockDim.x) {   // zero the upper triangle of the factor
-            const int i = e % D, j = e / D;
-            if (i < j) Lm[e] = 0.0;
-        }
+        double* xd = sh + BC::GT;          // diagonal of Y = L^-1
+        block_ldl_to_cholesky<DP>(sh, D, sh + BC::PIV, xd);
+        if ((int)threadIdx.x < DP) rows_tri_inverse<DP>(sh, D, xd, (int)threadIdx.x);
         __syncthreads();
-        block_tri_inverse(Lm, D);          // Lm now holds Y = L^-1 (lower)
+        auto Y = [&](int i, int j) { return i == j ? xd[i] : sh[i * BC::LD + j]; };   // j <= i
         // tau = tr(psi'^-1 P0) / nu' = sum over rows r of y_r^T P0 y_r / nu', P0 = nu0 psi0 + kappa0 m0 m0^T
         for (int rr = threadIdx.x; rr < D; rr += blockDim.x) {
             double acc = 0;
             if (psi0_identity) {
                 for (int a = 0; a <= rr; ++a) {
-                    const double y = Lm[(size_t)a * D + rr];
+                    const double y = Y(rr, a);
                     acc += y * y;
                 }
                 acc *= v0;
             } else {
                 double ym = 0;
                 for (int a = 0; a <= rr; ++a) {
-                    const double ya = Lm[(size_t)a * D + rr];
+                    const double ya = Y(rr, a);
                     ym += ya * m0[a];
                     double q = 0;
-                    for (int b = 0; b <= rr; ++b) q += psi0[(size_t)b * D + a] * Lm[(size_t)b * D + rr];
+                    for (int b = 0; b <= rr; ++b) q += psi0[(size_t)b * D + a] * Y(rr, b);
                     acc += ya * q;
                 }
                 acc = v0 * acc + k0 * ym * ym;
@@ -215,7 +214,10 @@ __global__ void __launch_bounds__(RegChol<DP>::T) k_screen_slots_niw(const doubl
         }
         tau = block_sum(tau, red) / vp;
         float* Li = linv + (size_t)(s / 3) * D * D;
-        for (int e = threadIdx.x; e < D * D; e += blockDim.x) Li[e] = (float)Lm[e];
+        for (int e = threadIdx.x; e < D * D; e += blockDim.x) {
+            const int i = e % D, j = e / D;
+            Li[e] = i < j ? 0.f : (float)Y(i, j);
+        }
     } else {
         h = block_sum(h, red);
         t = block_sum(t, red);
@@ -689,7 +691,7 @@ __global__ void __launch_bounds__(kTopThreads) k_screen_topk(const float* __rest
 // log marginal likelihood of the listed slots (the arithmetic of k_slot_lml), one block per slot
 // (sel, nullable: clusters whose slots use the second prior k1, v1, ld1, prior1 -- the outlier layout)
 template <int DP>
-__global__ void __launch_bounds__(RegChol<DP>::T) k_slot_lml_list(const double* __restrict__ stats, int stat_len, int D,
+__global__ void __launch_bounds__(BlockChol<DP>::T) k_slot_lml_list(const double* __restrict__ stats, int stat_len, int D,
                                                                    int gauss, double k0, double v0, double ld0,
                                                                    const double* __restrict__ prior, double k1,
                                                                    double v1, double ld1,
@@ -698,7 +700,7 @@ __global__ void __launch_bounds__(RegChol<DP>::T) k_slot_lml_list(const double* 
                                                                    const int32_t* __restrict__ slots,
                                                                    double* __restrict__ lml)
 {
-    __shared__ double sh[RegChol<DP>::SMEM];
+    extern __shared__ double sh[];
     const int s = slots[blockIdx.x];
     if (sel && sel[s / 3]) {
         k0 = k1;
@@ -709,16 +711,16 @@ __global__ void __launch_bounds__(RegChol<DP>::T) k_slot_lml_list(const double* 
     const double* st = stats + (size_t)s * stat_len;
     double v;
     if (gauss)
-        v = niw_lml_reg<DP>(D, st[0], st + 1, st + 1 + D, nullptr, nullptr, k0, v0, prior, prior + D, ld0, sh);
+        v = niw_lml_block<DP>(D, st[0], st + 1, st + 1 + D, nullptr, nullptr, k0, v0, prior, prior + D, ld0, sh);
     else
-        v = mult_lml_block(D, st[0], st + 1, nullptr, prior, sh + 3 * DP);
+        v = mult_lml_block(D, st[0], st + 1, nullptr, prior, sh + BlockChol<DP>::RED);
     if (threadIdx.x == 0) lml[s] = v;
 }
 
 // exact merge ratios of the listed pairs (the arithmetic of k_merge_hr), one block per pair; the merged
 // cluster takes cluster i's prior (shared_actions.cpp:88-95)
 template <int DP>
-__global__ void __launch_bounds__(RegChol<DP>::T) k_merge_hr_list(const double* __restrict__ stats, int stat_len, int D,
+__global__ void __launch_bounds__(BlockChol<DP>::T) k_merge_hr_list(const double* __restrict__ stats, int stat_len, int D,
                                                                    int gauss, double k0, double v0, double ld0,
                                                                    const double* __restrict__ prior, double k1,
                                                                    double v1, double ld1,
@@ -728,7 +730,7 @@ __global__ void __launch_bounds__(RegChol<DP>::T) k_merge_hr_list(const double* 
                                                                    const int32_t* __restrict__ pairs, double alpha,
                                                                    double* __restrict__ out)
 {
-    __shared__ double sh[RegChol<DP>::SMEM];
+    extern __shared__ double sh[];
     const int i = pairs[2 * blockIdx.x], j = pairs[2 * blockIdx.x + 1];
     if (sel && sel[i]) {
         k0 = k1;
@@ -736,7 +738,7 @@ __global__ void __launch_bounds__(RegChol<DP>::T) k_merge_hr_list(const double* 
         ld0 = ld1;
         prior = prior1;
     }
-    const double v = merge_log_hr_reg<DP>(stats, stat_len, D, gauss, k0, v0, ld0, prior, lml, i, j, alpha, sh);
+    const double v = merge_log_hr_block<DP>(stats, stat_len, D, gauss, k0, v0, ld0, prior, lml, i, j, alpha, sh);
     if (threadIdx.x == 0) out[blockIdx.x] = v;
 }
 
@@ -911,9 +913,9 @@ __global__ void k_mlp_adam(const float* __restrict__ part, int ntiles, float* __
 template <int DP>
 static dpmm_status launch_slots_niw(dpmm_ctx* c, int K)
 {
-    const size_t sm = sizeof(double) * (size_t)c->D * c->D;
+    constexpr size_t sm = BlockChol<DP>::bytes;
     DPMM_TRY(allow_smem(k_screen_slots_niw<DP>, sm));
-    k_screen_slots_niw<DP><<<3 * K, RegChol<DP>::T, sm, c->stream>>>(
+    k_screen_slots_niw<DP><<<3 * K, BlockChol<DP>::T, sm, c->stream>>>(
         c->d_stats, c->stat_len, c->D, c->prior_k, c->prior_v, c->prior_logdet, c->d_prior, c->prior_identity ? 1 : 0,
         c->d_scr_rec, c->d_scr_vec, c->d_scr_linv);
     return DPMM_OK;
@@ -988,12 +990,14 @@ dpmm_status launch_hastings_list(dpmm_ctx* c, int K, int kind, double alpha, int
     const bool out2 = c->outlier_layout != 0;
     const double* p2 = out2 ? c->d_prior2 : c->d_prior;
     const uint8_t* sel = out2 ? c->d_prior_sel : nullptr;
-    DPMM_WITH_DP(dp, (k_slot_lml_list<DP><<<nslots, RegChol<DP>::T, 0, c->stream>>>(
+    DPMM_WITH_DP(dp, DPMM_TRY(allow_smem(k_slot_lml_list<DP>, BlockChol<DP>::bytes));
+                 (k_slot_lml_list<DP><<<nslots, BlockChol<DP>::T, BlockChol<DP>::bytes, c->stream>>>(
                          c->d_stats, c->stat_len, c->D, gauss, c->prior_k, c->prior_v, c->prior_logdet, c->d_prior,
                          c->prior2_k, c->prior2_v, c->prior2_logdet, p2, sel, c->d_scr_slots, c->d_lml)));
     DPMM_LAUNCHED();
     if (kind == DPMM_SCREEN_MERGE) {
-        DPMM_WITH_DP(dp, (k_merge_hr_list<DP><<<n, RegChol<DP>::T, 0, c->stream>>>(
+        DPMM_WITH_DP(dp, DPMM_TRY(allow_smem(k_merge_hr_list<DP>, BlockChol<DP>::bytes));
+                 (k_merge_hr_list<DP><<<n, BlockChol<DP>::T, BlockChol<DP>::bytes, c->stream>>>(
                              c->d_stats, c->stat_len, c->D, gauss, c->prior_k, c->prior_v, c->prior_logdet, c->d_prior,
                              c->prior2_k, c->prior2_v, c->prior2_logdet, p2, sel, c->d_lml, c->d_scr_list, alpha,
                              c->d_scr_hr)));
