@@ -408,8 +408,11 @@ dpmm_status launch_cluster_labels(dpmm_ctx* c, int K, int final_, const float* d
 // chunk left with its own cluster only takes it as every point's label.
 constexpr int kPrTh = 128;       // threads per block
 
-// one block per cluster k: lam[k] = sqrt of the Gershgorin bound of lambda_max(W_k W_k^T) (inflated);
-// for every h: M[h][k] (deflated), v[h][k][DP] and beta[h][k]
+// blocks (cluster k, share of the clusters h): lam[k] = sqrt of the Gershgorin bound of lambda_max(W_k W_k^T)
+// (inflated; share 0); for every h of the share: M[h][k] (deflated), v[h][k][DP] and beta[h][k].  Bound by
+// shared-memory reads of W_k: kept as doubles (a conversion per multiply-add runs at a quarter of the FP64
+// rate), one read serves HB clusters h, and the shares fill the device where K alone does not (K = 100,
+// D = 64: 85 -> 31 us; K = 20, D = 32: 11.8 -> 6.9 us).
 template <int DP>
 __global__ void __launch_bounds__(kPrTh) k_prune_prep(const float* __restrict__ Wt, const float* __restrict__ mu,
                                                       int K, float* __restrict__ lam, float* __restrict__ M,
@@ -419,25 +422,25 @@ __global__ void __launch_bounds__(kPrTh) k_prune_prep(const float* __restrict__ 
     constexpr int SW = DP + 1;   // padded row stride: the z loop's lanes read one column each
     constexpr int TPR = kPrTh / DP < DP ? kPrTh / DP : DP;   // threads per Gershgorin row (each >= 1 column)
     static_assert(kPrTh % DP == 0 && DP % TPR == 0, "row split");
-    __shared__ float sW[DP * SW];
+    __shared__ double sW[DP * SW];
     __shared__ double red[NW];
     __shared__ double srow_part[kPrTh];
-    __shared__ double zs[NW][DP];
-    __shared__ double dm[NW][DP];
+    constexpr int HB = 4, ZP = (DP + 31) / 32;
+    __shared__ double dm[NW][HB][DP];
     const int k = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    for (int e = t; e < DP * DP; e += blockDim.x) sW[(e / DP) * SW + e % DP] = Wt[(size_t)3 * k * DP * DP + e];
+    for (int e = t; e < DP * DP; e += blockDim.x) sW[(e / DP) * SW + e % DP] = (double)Wt[(size_t)3 * k * DP * DP + e];
     __syncthreads();
-    if (t < DP * TPR) {   // Gershgorin row sums of W W^T: row t % DP, column share t / DP, four chains
+    if (blockIdx.y == 0 && t < DP * TPR) {   // Gershgorin row sums of W W^T: row t % DP, column share t / DP, four chains
         const int i = t % DP, j0 = (t / DP) * (DP / TPR);
         double srow = 0;
         for (int j = j0; j < j0 + DP / TPR; ++j) {
             double l0 = 0, l1 = 0, l2 = 0, l3 = 0;
 #pragma unroll
             for (int cc = 0; cc < DP; cc += 4) {
-                l0 = fma((double)sW[cc * SW + i], (double)sW[cc * SW + j], l0);
-                l1 = fma((double)sW[(cc + 1) * SW + i], (double)sW[(cc + 1) * SW + j], l1);
-                l2 = fma((double)sW[(cc + 2) * SW + i], (double)sW[(cc + 2) * SW + j], l2);
-                l3 = fma((double)sW[(cc + 3) * SW + i], (double)sW[(cc + 3) * SW + j], l3);
+                l0 = fma(sW[cc * SW + i], sW[cc * SW + j], l0);
+                l1 = fma(sW[(cc + 1) * SW + i], sW[(cc + 1) * SW + j], l1);
+                l2 = fma(sW[(cc + 2) * SW + i], sW[(cc + 2) * SW + j], l2);
+                l3 = fma(sW[(cc + 3) * SW + i], sW[(cc + 3) * SW + j], l3);
             }
             srow += fabs((l0 + l1) + (l2 + l3));
         }
@@ -445,7 +448,7 @@ __global__ void __launch_bounds__(kPrTh) k_prune_prep(const float* __restrict__ 
     }
     __syncthreads();
     double rmax = 0;
-    if (t < DP) {
+    if (blockIdx.y == 0 && t < DP) {
         double tot = 0;
         for (int p = 0; p < TPR; ++p) tot += srow_part[t + p * DP];
         rmax = tot;
@@ -454,55 +457,94 @@ __global__ void __launch_bounds__(kPrTh) k_prune_prep(const float* __restrict__ 
     for (int o = 16; o; o >>= 1) rmax = fmax(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
     if (lane == 0) red[warp] = rmax;
     __syncthreads();
-    if (t == 0) {
+    if (blockIdx.y == 0 && t == 0) {
         double m = 0;
         for (int w = 0; w < NW; ++w) m = fmax(m, red[w]);
         lam[k] = (float)(sqrt(m) * (1.0 + 1e-5));
     }
     const float* mk = mu + (size_t)3 * k * DP;
-    for (int h = warp; h < K; h += NW) {
-        const float* mh = mu + (size_t)3 * h * DP;
-        for (int i = lane; i < DP; i += 32) dm[warp][i] = (double)mh[i] - (double)mk[i];
-        __syncwarp();
-        double q = 0;
-        for (int j = lane; j < DP; j += 32) {   // z = W_k^T (mu_h - mu_k)
-            double z0 = 0, z1 = 0, z2 = 0, z3 = 0;
+    // a warp takes HB clusters h at a time: one read of W_k serves HB multiply-adds
+    for (int h0 = (blockIdx.y * NW + warp) * HB; h0 < K; h0 += gridDim.y * NW * HB) {
+        double(*dz)[DP] = dm[warp];   // mu_h - mu_k, then z
 #pragma unroll
-            for (int i = 0; i < DP; i += 4) {
-                z0 = fma((double)sW[j * SW + i], dm[warp][i], z0);
-                z1 = fma((double)sW[j * SW + i + 1], dm[warp][i + 1], z1);
-                z2 = fma((double)sW[j * SW + i + 2], dm[warp][i + 2], z2);
-                z3 = fma((double)sW[j * SW + i + 3], dm[warp][i + 3], z3);
+        for (int q = 0; q < HB; ++q) {
+            const float* mh = mu + (size_t)3 * min(h0 + q, K - 1) * DP;
+            for (int i = lane; i < DP; i += 32) dz[q][i] = (double)mh[i] - (double)mk[i];
+        }
+        __syncwarp();
+        double zz[ZP][HB], nz[HB], inv[HB];
+#pragma unroll
+        for (int q = 0; q < HB; ++q) nz[q] = 0;
+#pragma unroll
+        for (int p = 0; p < ZP; ++p) {   // z = W_k^T (mu_h - mu_k)
+            const int j = lane + 32 * p;
+            if (j >= DP) continue;
+            double z[HB][4];
+#pragma unroll
+            for (int q = 0; q < HB; ++q)
+#pragma unroll
+                for (int m = 0; m < 4; ++m) z[q][m] = 0;
+#pragma unroll 2
+            for (int i = 0; i < DP; i += 4)
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const double w = sW[j * SW + i + m];
+#pragma unroll
+                    for (int q = 0; q < HB; ++q) z[q][m] = fma(w, dz[q][i + m], z[q][m]);
+                }
+#pragma unroll
+            for (int q = 0; q < HB; ++q) {
+                zz[p][q] = (z[q][0] + z[q][1]) + (z[q][2] + z[q][3]);
+                nz[q] += zz[p][q] * zz[p][q];
             }
-            const double z = (z0 + z1) + (z2 + z3);
-            zs[warp][j] = z;
-            q += z * z;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < HB; ++q) {
+#pragma unroll
+            for (int p = 0; p < ZP; ++p)
+                if (lane + 32 * p < DP) dz[q][lane + 32 * p] = zz[p][q];
+#pragma unroll
+            for (int o = 16; o; o >>= 1) nz[q] += __shfl_xor_sync(0xffffffffu, nz[q], o);
+            nz[q] = sqrt(nz[q]);
+            inv[q] = nz[q] > 0 ? 1.0 / nz[q] : 0.0;
+        }
+        __syncwarp();
+        double bsum[HB];
+#pragma unroll
+        for (int q = 0; q < HB; ++q) bsum[q] = 0;
+#pragma unroll
+        for (int p = 0; p < ZP; ++p) {    // v = W_k u, u = z / |z|
+            const int i = lane + 32 * p;
+            if (i >= DP) continue;
+            double v[HB][4];
+#pragma unroll
+            for (int q = 0; q < HB; ++q)
+#pragma unroll
+                for (int m = 0; m < 4; ++m) v[q][m] = 0;
+#pragma unroll 2
+            for (int j = 0; j < DP; j += 4)
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const double w = sW[(j + m) * SW + i];
+#pragma unroll
+                    for (int q = 0; q < HB; ++q) v[q][m] = fma(w, dz[q][j + m], v[q][m]);
+                }
+#pragma unroll
+            for (int q = 0; q < HB; ++q) {
+                const double vv = ((v[q][0] + v[q][1]) + (v[q][2] + v[q][3])) * inv[q];
+                if (h0 + q < K) V[((size_t)(h0 + q) * K + k) * DP + i] = (float)vv;
+                bsum[q] += (double)(float)vv * (double)mk[i];
+            }
         }
 #pragma unroll
-        for (int o = 16; o; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-        __syncwarp();
-        const double nz = sqrt(q);
-        const double inv = nz > 0 ? 1.0 / nz : 0.0;
-        float* vh = V + ((size_t)h * K + k) * DP;
-        double bsum = 0;
-        for (int i = lane; i < DP; i += 32) {    // v = W_k u, u = z / |z|
-            double v0 = 0, v1 = 0, v2 = 0, v3 = 0;
+        for (int q = 0; q < HB; ++q) {
 #pragma unroll
-            for (int j = 0; j < DP; j += 4) {
-                v0 = fma((double)sW[j * SW + i], zs[warp][j], v0);
-                v1 = fma((double)sW[(j + 1) * SW + i], zs[warp][j + 1], v1);
-                v2 = fma((double)sW[(j + 2) * SW + i], zs[warp][j + 2], v2);
-                v3 = fma((double)sW[(j + 3) * SW + i], zs[warp][j + 3], v3);
+            for (int o = 16; o; o >>= 1) bsum[q] += __shfl_xor_sync(0xffffffffu, bsum[q], o);
+            if (lane == 0 && h0 + q < K) {
+                M[(size_t)(h0 + q) * K + k] = (float)(nz[q] * (1.0 - 1e-5));
+                beta[(size_t)(h0 + q) * K + k] = (float)bsum[q];
             }
-            const double v = ((v0 + v1) + (v2 + v3)) * inv;
-            vh[i] = (float)v;
-            bsum += (double)(float)v * (double)mk[i];
-        }
-#pragma unroll
-        for (int o = 16; o; o >>= 1) bsum += __shfl_xor_sync(0xffffffffu, bsum, o);
-        if (lane == 0) {
-            M[(size_t)h * K + k] = (float)(nz * (1.0 - 1e-5));
-            beta[(size_t)h * K + k] = (float)bsum;
         }
         __syncwarp();
     }
@@ -757,7 +799,8 @@ template <int DP>
 static dpmm_status launch_pruned_dp(dpmm_ctx* c, int K, int final_, const float* d_u, bool tc_dense, bool* used)
 {
     DPMM_TRY(build_permutation(c, K));
-    k_prune_prep<DP><<<K, kPrTh, 0, c->stream>>>(c->d_Wt, c->d_mu, K, c->d_prune_lam, c->d_prune_M, c->d_prune_V,
+    const dim3 pgrid((unsigned)K, (unsigned)std::max(1, std::min((K + 15) / 16, 5 * c->num_sms / K)));   // up to five blocks per SM, 16 h per pass
+    k_prune_prep<DP><<<pgrid, kPrTh, 0, c->stream>>>(c->d_Wt, c->d_mu, K, c->d_prune_lam, c->d_prune_M, c->d_prune_V,
                                                  c->d_prune_beta);
     DPMM_LAUNCHED();
     DPMM_CUDA_TRY(cudaMemsetAsync(c->d_prune_cnt, 0, 2 * sizeof(unsigned long long), c->stream));
