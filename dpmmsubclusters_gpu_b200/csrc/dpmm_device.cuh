@@ -176,16 +176,20 @@ struct AliasAcc {
     int stride;
 };
 
-// Two-category draw used by the sub-cluster phase: the general construction with n = 2 on
-// a 4-entry table, with the reference's float->double promotions replaced by float maths.
-__device__ __forceinline__ int alias_draw2(float p1, float p2, float u1, float u2)
+// Two-category draw of the sub-cluster phase from rl, rr = log-likelihood + log weight of both sides: the
+// 2-way softmax (cudaKernel.cu:352-372) and the general alias construction for n = 2, with the
+// reference's float->double promotions replaced by float maths.  Of the two exponentials one is exp(0) = 1
+// and the other e <= 1, s = 1 + e their sum.  Only the smaller category, y = 2 e / s < 1, can go to the other,
+// and only when that one has an excess (2 / s > 1, that is s < 2); a larger one drawn keeps itself.  The
+// column of the first uniform (alias_column for n = 2) is 2 from the first float above 1 / 1.999999 on.
+__device__ __forceinline__ int draw_sub_label(float rl, float rr, float u1, float u2)
 {
-    float y[4];
-    uint8_t a[4], b[4];
-    y[1] = p1 * 2.0f;
-    y[2] = p2 * 2.0f;
-    AliasAcc<float, uint8_t> acc{y, a, b, 1};
-    return alias_draw<float, uint8_t>(2, acc, u1, u2);
+    const int col = u1 >= 0.50000029802322388f ? 2 : 1;
+    const bool l_larger = rl >= rr;
+    if ((col == 1) == l_larger) return col;
+    const float e = __expf(-fabsf(rl - rr)), s = 1.0f + e;
+    const float y = (e / s) * 2.0f;
+    return s < 2.0f && y < 1.0f && y < u2 ? 3 - col : col;
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -136,7 +136,9 @@ struct dpmm_ctx {
     uint8_t* d_Atc = nullptr;      // tensor-core A operand: per 128 points the same 32 KB split-bf16
                                    // swizzled tile, packed once when the points are uploaded
     uint8_t* d_Bsub = nullptr;     // tensor-core sub-label phase: per cluster its two sub-cluster
-                                   // factors as one 32 KB split-bf16 swizzled B tile
+                                   // factors as one 32 KB split-bf16 swizzled B tile (Dp = 32: the fused
+                                   // sub-label + statistics pass only, packed while it is on)
+    uint8_t* d_Bsub32 = nullptr;   // ... at Dp = 32: per cluster 64 rows of [32 hi | 32 lo], 8 KB
     uint8_t* d_Amult = nullptr;    // multinomial tensor-core label phase: the counts as BF16, per
                                    // (128-point tile, 64-category block) one 16 KB swizzled tile
     uint8_t* d_Bmult = nullptr;    // ... log theta of the clusters as three BF16 parts per block
@@ -364,10 +366,11 @@ dpmm_status pack_mult_tc_points(dpmm_ctx* c);          // the counts as BF16 til
 dpmm_status pack_mult_tc_params(dpmm_ctx* c, int K);   // log theta as three BF16 parts
 dpmm_status launch_mult_labels_tc(dpmm_ctx* c, int K, int final_, const float* d_u, float* d_rout);
 size_t tc_param_bytes(int k_max);          // B tiles + bias records for k_max clusters
-// tensor-core sub-label kernel (dpmm_tc.cu): draws the sub-labels only (statistics separately)
+// tensor-core sub-label kernel (dpmm_rows_tc.cu): draws the sub-labels only (statistics separately)
 bool tc_sub_supported(const dpmm_ctx* c);
 // defer_check: its error word is read by the statistics launch that follows (one sync for both)
 dpmm_status launch_sub_labels_tc(dpmm_ctx* c, RngArgs r, float* d_rout, bool defer_check = false);
+dpmm_status pack_sub32_params(dpmm_ctx* c, int K);   // its B operand at Dp = 32
 // pass 1 of the pruned label phase on the tensor cores (dpmm_tc.cu; Dp = 32 or 64, packed B tiles)
 bool tc_scan_supported(const dpmm_ctx* c, int K);
 dpmm_status launch_prune_scan_tc(dpmm_ctx* c, int K, int32_t* d_err);

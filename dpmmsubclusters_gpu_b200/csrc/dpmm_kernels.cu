@@ -1326,12 +1326,9 @@ __global__ void __launch_bounds__(256, (DP >= 128 ? 1 : 2)) k_gauss_sub_stats(
                 // + log lr_weights, then the 2-way softmax (cudaKernel.cu:352-372)
                 rl += wl;
                 rr += wr;
-                float mx = fmaxf(rl, rr);
-                float el = __expf(rl - mx), er = __expf(rr - mx);
-                float s = el + er;
                 float u1, u2;
                 draw_uniform2(rng, pt, u1, u2);
-                sv = alias_draw2(el / s, er / s, u1, u2);
+                sv = draw_sub_label(rl, rr, u1, u2);
                 sub[pt] = sv;
             } else {
                 sv = sub[pt];
@@ -1682,12 +1679,9 @@ __global__ void __launch_bounds__(256) k_mult_sub_stats(
             if (lane == 0) {
                 float rl = dl + wl, rr = dr + wr;
                 if (r_out) { r_out[2 * pt] = dl; r_out[2 * pt + 1] = dr; }
-                float mx = fmaxf(rl, rr);
-                float el = __expf(rl - mx), er = __expf(rr - mx);
-                float s = el + er;
                 float u1, u2;
                 draw_uniform2(rng, pt, u1, u2);
-                sv = alias_draw2(el / s, er / s, u1, u2);
+                sv = draw_sub_label(rl, rr, u1, u2);
                 sub[pt] = sv;
             }
             sv = __shfl_sync(0xffffffffu, lane == 0 ? sv : 0, 0);

@@ -22,23 +22,17 @@
 // stored at chunk c ^ (r % 8)), descriptor SBO = 1024 B; a K-step of 16 elements advances the
 // descriptor start address by 32 bytes.  The padded dimension must be 32 or 64 (zero-filled
 // to 64).
-#include <cuda_bf16.h>
-
 #include <algorithm>
 
-#include "dpmm_device.cuh"
+#include "dpmm_tc.cuh"
 
 namespace dpmm {
 namespace tc {
 
-constexpr int BM = 128;                    // points per tile (TMEM lanes)
-constexpr int KD = 64;                     // contraction length (one 128-byte bf16 row)
 constexpr int CPT = 2;                     // clusters per N tile
 constexpr int BN = CPT * KD;               // 128 accumulator columns per N tile
-constexpr int A_BYTES = BM * KD * 2;       // 16 KB (one of hi / lo)
 constexpr int B_BYTES = BN * KD * 2;       // 16 KB (one of hi / lo)
 constexpr int STAGE_BYTES = 2 * B_BYTES;   // 32 KB: hi then lo
-constexpr int A_TILE = 2 * A_BYTES;        // 32 KB: hi then lo
 constexpr uint32_t TMEM_COLS = 512;        // 2 accumulator pairs: 2 halves x 128 columns each
 constexpr int NPAIR = 2;                   // accumulator pairs (N tiles in flight)
 constexpr int HALVES = 2;                  // point tiles per super-tile (M = 2 x 128 per B tile)
@@ -51,199 +45,10 @@ constexpr int DRAIN_WARPS = 16;            // (lane quarter, cluster of the N ti
 constexpr int WARP_MMA0 = 1, WARP_DRAIN0 = WARP_MMA0 + MMA_WARPS;
 constexpr int THREADS = 32 * (1 + MMA_WARPS + DRAIN_WARPS);
 
-enum : int {
-    ERR_TIMEOUT_FULL = 1, ERR_TIMEOUT_EMPTY = 2, ERR_TIMEOUT_TFULL = 3, ERR_TIMEOUT_TEMPTY = 4,
-    ERR_TIMEOUT_AFULL = 5, ERR_TIMEOUT_AEMPTY = 6, ERR_TIMEOUT_BFULL = 9, ERR_TIMEOUT_BEMPTY = 10
-};
-
-__host__ __device__ constexpr uint32_t sw128_offset(int row, int k)
-{
-    return (uint32_t)((row >> 3) * 1024 + (row & 7) * 128 + ((((k >> 3) ^ (row & 7)) & 7) << 4) + (k & 7) * 2);
-}
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-__device__ __forceinline__ uint64_t global_ns()
-{
-    uint64_t t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-
-constexpr uint64_t WAIT_LIMIT_NS = 2000000000ull;   // 2 s: legitimate waits here are microseconds
-
-// Non-blocking probe of a phase (no suspend).
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-// Potentially blocking probe: the thread may sleep until the phase completes, for at most about
-// `ns` nanoseconds (the suspend-time hint), instead of returning at once and spinning.
-__device__ __forceinline__ bool mbar_try_wait_sleep(uint64_t* bar, uint32_t parity, uint32_t ns)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(ns)
-        : "memory");
-    return ok != 0;
-}
-
-// Single-thread bounded wait.  Gives up after WAIT_LIMIT_NS, or early when another CTA of the
-// launch has already reported an error (gerr != nullptr).  Between non-blocking probes the thread
-// backs off with nanosleep (32 ns growing to 256 ns), so that waiting warps do not fill the issue
-// slots and the barrier / timer pipes that the working warps need.
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, const volatile int32_t* gerr)
-{
-    if (mbar_test_wait(bar, parity)) return true;
-    const uint64_t t0 = global_ns();
-    uint32_t sleep = 32;
-    for (uint32_t i = 1;; ++i) {
-        __nanosleep(sleep);
-        if (mbar_test_wait(bar, parity)) return true;
-        if (sleep < 256) sleep <<= 1;
-        if ((i & 63) == 0) {
-            if (global_ns() - t0 > WAIT_LIMIT_NS) return false;
-            if (gerr && *gerr) return false;
-        }
-    }
-}
-
-// Warp-uniform bounded wait: lane 0 polls (one barrier operation per poll instead of 32) and
-// the outcome is broadcast; __syncwarp orders the other lanes after lane 0's acquire.  All lanes
-// take the same decision (the epilogue's tcgen05.ld is warp-collective).
-__device__ __forceinline__ bool warp_wait_bounded(uint64_t* bar, uint32_t parity, const volatile int32_t* gerr)
-{
-    int ok = 1;
-    if ((threadIdx.x & 31) == 0) ok = mbar_wait_bounded(bar, parity, gerr) ? 1 : 0;
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    __syncwarp();
-    return ok != 0;
-}
-
-// One arrival per warp: every lane's prior work is ordered before lane 0's release by __syncwarp.
-__device__ __forceinline__ void warp_arrive(uint64_t* bar)
-{
-    __syncwarp();
-    if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
-}
-
-__device__ __forceinline__ void bulk_copy_g2s(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar)
-{
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_u32(smem_dst)),
-        "l"(gmem_src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
-
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr)
-{
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);   // start address
-    d |= (uint64_t)1 << 16;                      // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;            // stride byte offset: 8-row atoms 1024 B apart
-    d |= (uint64_t)1 << 46;                      // descriptor version (sm_100)
-    d |= (uint64_t)2 << 61;                      // 128-byte swizzle
-    return d;
-}
-
-// kind::f16 instruction descriptor: F32 accumulator, BF16 A and B, both K-major, M=128, N=128
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accum)
 {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accum)
-        : "memory");
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t* bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-                 : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// 32 consecutive accumulator columns of this thread's TMEM lane (warp-collective)
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32])
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void bf16_split(float v, __nv_bfloat16& hi, __nv_bfloat16& lo)
-{
-    hi = __float2bfloat16_rn(v);
-    lo = __float2bfloat16_rn(v - __bfloat162float(hi));
-}
-
-__device__ __forceinline__ uint32_t bf16x2_bits(__nv_bfloat162 v)
-{
-    return (uint32_t)__bfloat16_as_ushort(v.x) | ((uint32_t)__bfloat16_as_ushort(v.y) << 16);
-}
-
-// bf16_split of four values, packed: hi and lo as 4 x BF16 (8 bytes) each
-__device__ __forceinline__ void bf16_split4(float a, float b, float c, float d, uint2& hi, uint2& lo)
-{
-    const __nv_bfloat162 h01 = __floats2bfloat162_rn(a, b), h23 = __floats2bfloat162_rn(c, d);
-    const float2 f01 = __bfloat1622float2(h01), f23 = __bfloat1622float2(h23);
-    hi = make_uint2(bf16x2_bits(h01), bf16x2_bits(h23));
-    lo = make_uint2(bf16x2_bits(__floats2bfloat162_rn(a - f01.x, b - f01.y)),
-                    bf16x2_bits(__floats2bfloat162_rn(c - f23.x, d - f23.y)));
+    umma_bf16_n(tmem_d, adesc, bdesc, bf16_idesc(BN), accum);
 }
 
 // ------------------------------------------------------------------------- B packing
@@ -647,201 +452,6 @@ __global__ void __launch_bounds__(256) k_draw_labels(const float* __restrict__ r
     float u1, u2;
     draw_uniform2(rng, pt, u1, u2);
     labels[pt] = alias_draw_y(y, is_small, K, u1, u2);
-}
-
-// ------------------------------------------------------------------------- sub-label kernel
-// Sub-cluster labels of the points of one chunk (one cluster, in label order; cudaKernel.cu
-// create_subclusters_labels, :1299-1398): per tile of 128 points the A operand (split BF16,
-// swizzled) is built in shared memory from the gathered rows, and 12 tcgen05.mma against the
-// cluster's B tile [W_l | W_r] give z for both sub-clusters.  8 warps drain
-// r_s = c_s - |z_s - b_s|^2 / 2 (warp w: lane quarter w % 4, side w / 4); one thread per point then
-// adds log lr_weights, normalises and draws with the two-category alias (cudaKernel.cu:352-372).
-// Every wait is bounded and decided block-uniformly.
-struct SubSmem {
-    static constexpr size_t b = 0;                        // 32 KB B tile (hi, lo)
-    static constexpr size_t a = STAGE_BYTES;              // 32 KB A tile (hi, lo)
-    static constexpr size_t q = a + A_TILE;               // r of both sides [2][BM] floats
-    static constexpr size_t bias = q + 2 * BM * 4;        // b_l, b_r [2][KD] floats
-    static constexpr size_t pidx = bias + 2 * KD * 4;     // the tile's permutation entries [2][BM] ints
-    static constexpr size_t bar = pidx + 2 * BM * 4;      // mbarrier, tmem slot, flag
-    static constexpr size_t total = bar + 32 + 1024;      // + alignment slack
-};
-
-template <int DP>
-__global__ void __launch_bounds__(256, 2) k_sub_labels_tc(
-    const float* __restrict__ x, const int32_t* __restrict__ perm, const int32_t* __restrict__ chunk,
-    const int32_t* __restrict__ nchunks, const uint8_t* __restrict__ Bsub, const float* __restrict__ bvec,
-    const float* __restrict__ cvec, const float* __restrict__ lrw, RngArgs rng, int32_t* __restrict__ sub,
-    float* __restrict__ r_out, int32_t* __restrict__ err, int stall)
-{
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t* sB = smem + SubSmem::b;
-    uint8_t* sA = smem + SubSmem::a;
-    float* sq = reinterpret_cast<float*>(smem + SubSmem::q);
-    float* sbias = reinterpret_cast<float*>(smem + SubSmem::bias);
-    int32_t* spidx = reinterpret_cast<int32_t*>(smem + SubSmem::pidx);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + SubSmem::bar);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 1);
-    volatile int* flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-
-    const int ch = blockIdx.x;
-    if (ch >= *nchunks) return;
-    const int k = chunk[3 * ch], start = chunk[3 * ch + 1], len = chunk[3 * ch + 2];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const volatile int32_t* gerr = err;
-
-    // B tile of cluster k and the two sub-cluster biases
-    {
-        const uint4* src = reinterpret_cast<const uint4*>(Bsub + (size_t)k * STAGE_BYTES);
-        uint4* dst = reinterpret_cast<uint4*>(sB);
-        for (int e = tid; e < STAGE_BYTES / 16; e += 256) dst[e] = src[e];
-        if (tid < 2 * KD) {
-            const int side = tid / KD, j = tid % KD;
-            sbias[tid] = j < DP ? bvec[(size_t)(3 * k + 1 + side) * DP + j] : 0.f;
-        }
-    }
-    if (tid == 0) {
-        mbar_init(bar, 1);
-        *flag = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"((uint32_t)BN));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
-    const float cl = cvec[3 * k + 1], cr = cvec[3 * k + 2];
-    const float wl = lrw[2 * k], wr = lrw[2 * k + 1];
-
-    // gathered rows: item u of this thread is (row tid / 8 + 32 u, 8-float chunk tid % 8); a tile's
-    // permutation entries load one tile ahead of its rows
-    float4 pf[4][2];
-    int pq[4], pcur[4];   // entries of the tile after the loaded one / of the loaded one
-    auto load_perm = [&](int t0) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int row = (tid >> 3) + 32 * u;
-            pq[u] = t0 + row < len ? __ldg(perm + start + t0 + row) : -1;
-        }
-    };
-    auto load_rows = [&]() {   // rows of the tile whose entries pq holds
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int c8 = tid & 7;
-            pcur[u] = pq[u];
-            pf[u][0] = make_float4(0.f, 0.f, 0.f, 0.f);
-            pf[u][1] = pf[u][0];
-            if (pq[u] >= 0 && c8 * 8 < DP) {
-                const float4* src = reinterpret_cast<const float4*>(x + (size_t)pq[u] * DP + c8 * 8);
-                pf[u][0] = __ldg(src);
-                pf[u][1] = __ldg(src + 1);
-            }
-        }
-    };
-    load_perm(0);
-    load_rows();
-    load_perm(BM);
-    uint32_t phase = 0;
-    bool failed = false;
-    const uint64_t da_h = sw128_desc(smem_u32(sA)), da_l = sw128_desc(smem_u32(sA + A_BYTES));
-    const uint64_t db_h = sw128_desc(smem_u32(sB)), db_l = sw128_desc(smem_u32(sB + B_BYTES));
-    for (int t0 = 0; t0 < len && !failed; t0 += BM) {
-        const int nt = min(BM, len - t0);
-        // A tile: split BF16, 128-byte swizzle
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int row = (tid >> 3) + 32 * u, c8 = tid & 7;
-            const float v[8] = {pf[u][0].x, pf[u][0].y, pf[u][0].z, pf[u][0].w,
-                                pf[u][1].x, pf[u][1].y, pf[u][1].z, pf[u][1].w};
-            __align__(16) __nv_bfloat16 hi[8], lo[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) bf16_split(v[q], hi[q], lo[q]);
-            const uint32_t off = sw128_offset(row, c8 * 8);
-            *reinterpret_cast<uint4*>(sA + off) = *reinterpret_cast<const uint4*>(hi);
-            *reinterpret_cast<uint4*>(sA + A_BYTES + off) = *reinterpret_cast<const uint4*>(lo);
-            if (c8 == 0) spidx[((t0 / BM) & 1) * BM + row] = pcur[u];   // for the draw, two tiles apart
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        tc_fence_before();
-        __syncthreads();
-        if (tid == 0 && !stall) {   // stall: the wait-test seam issues nothing
-            tc_fence_after();
-#pragma unroll
-            for (int ks = 0; ks < KD / 16; ++ks) umma_bf16(tmem_base, da_h + 2 * ks, db_h + 2 * ks, ks != 0 ? 1u : 0u);
-#pragma unroll
-            for (int ks = 0; ks < KD / 16; ++ks) umma_bf16(tmem_base, da_l + 2 * ks, db_h + 2 * ks, 1u);
-#pragma unroll
-            for (int ks = 0; ks < KD / 16; ++ks) umma_bf16(tmem_base, da_h + 2 * ks, db_l + 2 * ks, 1u);
-            umma_commit(bar);
-        }
-        if (t0 + BM < len) {   // the next tile's rows load while the MMAs run
-            load_rows();
-            load_perm(t0 + 2 * BM);
-        }
-        if (tid == 0) {
-            if (!mbar_wait_bounded(bar, phase & 1, gerr)) {
-                atomicCAS(err, 0, ERR_TIMEOUT_TFULL);
-                *flag = 1;
-            }
-        }
-        ++phase;
-        __syncthreads();
-        if (*flag) { failed = true; break; }
-        tc_fence_after();
-        {
-            const int quarter = warp & 3, side = warp >> 2;
-            const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-            const float* bs = sbias + side * KD;
-            float q0 = 0.f, q1 = 0.f, q2 = 0.f, q3 = 0.f;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                if (h == 1 && DP <= 32) break;   // columns past DP are zero
-                uint32_t v[32];
-                tmem_ld32(tmem_base + lane_addr + (uint32_t)(side * KD + 32 * h), v);
-#pragma unroll
-                for (int j4 = 0; j4 < 8; ++j4) {
-                    const float4 b4 = *reinterpret_cast<const float4*>(bs + 32 * h + 4 * j4);
-                    const float z0 = __uint_as_float(v[4 * j4 + 0]) - b4.x;
-                    const float z1 = __uint_as_float(v[4 * j4 + 1]) - b4.y;
-                    const float z2 = __uint_as_float(v[4 * j4 + 2]) - b4.z;
-                    const float z3 = __uint_as_float(v[4 * j4 + 3]) - b4.w;
-                    q0 = fmaf(z0, z0, q0);
-                    q1 = fmaf(z1, z1, q1);
-                    q2 = fmaf(z2, z2, q2);
-                    q3 = fmaf(z3, z3, q3);
-                }
-            }
-            sq[side * BM + quarter * 32 + lane] = (side ? cr : cl) - 0.5f * ((q0 + q1) + (q2 + q3));
-        }
-        tc_fence_before();
-        __syncthreads();
-        if (tid < nt) {
-            const int64_t pt = spidx[((t0 / BM) & 1) * BM + tid];
-            float rl = sq[tid], rr = sq[BM + tid];
-            if (r_out) { r_out[2 * pt] = rl; r_out[2 * pt + 1] = rr; }
-            rl += wl;
-            rr += wr;
-            const float mx = fmaxf(rl, rr);
-            const float el = __expf(rl - mx), er = __expf(rr - mx);
-            const float s = el + er;
-            float u1, u2;
-            draw_uniform2(rng, pt, u1, u2);
-            sub[pt] = alias_draw2(el / s, er / s, u1, u2);
-        }
-    }
-    if (failed && tid == 0 && !stall) mbar_wait_bounded(bar, (phase - 1) & 1, nullptr);   // nothing in flight at dealloc
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 0) {
-        tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)BN));
-    }
 }
 
 // ------------------------------------------------------------------------- pruned-phase scan
@@ -2258,12 +1868,9 @@ __global__ void __launch_bounds__(SS_THREADS, 1) k_sub_stats_tc(
                 }
                 rl += wl;
                 rr += wr;
-                const float mx = fmaxf(rl, rr);
-                const float el = __expf(rl - mx), er = __expf(rr - mx);
-                const float s = el + er;
                 float u1, u2;
                 draw_uniform2(rng, pt, u1, u2);
-                lab = alias_draw2(el / s, er / s, u1, u2);
+                lab = draw_sub_label(rl, rr, u1, u2);
                 sub[pt] = lab;
             }
             ssub[slot * SS_T + p] = lab;
@@ -2398,13 +2005,11 @@ __global__ void __launch_bounds__(SS_THREADS, 1) k_sub_stats_tc(
 
 }  // namespace tc
 
-constexpr size_t kTcSmemCap = 227 * 1024;
-
 // B stages: the deepest ring that fits
 static bool tc_config(int& bstages)
 {
     for (int bs = tc::MAX_BSTAGES; bs >= 2; --bs)
-        if (tc::smem_layout(bs).total <= kTcSmemCap) {
+        if (tc::smem_layout(bs).total <= tc::kTcSmemCap) {
             bstages = bs;
             return true;
         }
@@ -2436,7 +2041,8 @@ dpmm_status pack_tc_params(dpmm_ctx* c, int K)
     const int total = NT * tc::BN * 8;
     tc::k_pack_b<<<(total + 255) / 256, 256, 0, c->stream>>>(c->d_Wt, K, c->Dp, NT, 0, c->d_Btc);
     DPMM_LAUNCHED();
-    if (c->d_Bsub) {
+    if (c->d_Bsub32) DPMM_TRY(pack_sub32_params(c, K));
+    if (c->d_Bsub && (c->Dp == 64 || c->fuse_sub_stats)) {
         const int ts = K * tc::BN * 8;
         tc::k_pack_b<<<(ts + 255) / 256, 256, 0, c->stream>>>(c->d_Wt, K, c->Dp, K, 1, c->d_Bsub);
         DPMM_LAUNCHED();
@@ -2485,42 +2091,6 @@ dpmm_status launch_cluster_labels_tc(dpmm_ctx* c, int K, int final_, const float
     DPMM_CUDA_TRY(cudaMemcpyAsync(&h_err, err, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
     DPMM_CUDA_TRY(cudaStreamSynchronize(c->stream));
     if (h_err) return fail(DPMM_ERR_TIMEOUT, "tensor-core label kernel: bounded wait expired (code " +
-                                                 std::to_string(h_err) + ")");
-    return DPMM_OK;
-}
-
-bool tc_sub_supported(const dpmm_ctx* c)
-{
-    return c->prior == DPMM_PRIOR_GAUSSIAN && c->d_Bsub != nullptr && (c->Dp == 32 || c->Dp == 64) &&
-           c->ll_mode != DPMM_LL_FP32;
-}
-
-template <int DP>
-static dpmm_status launch_sub_labels_tc_t(dpmm_ctx* c, RngArgs r, float* d_rout, int32_t* err)
-{
-    auto kern = tc::k_sub_labels_tc<DP>;
-    DPMM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::SubSmem::total));
-    kern<<<c->max_chunks, 256, tc::SubSmem::total, c->stream>>>(c->d_x, c->d_perm, c->d_chunk, c->d_nchunks, c->d_Bsub,
-                                                              c->d_b, c->d_c, c->d_lrw, r, c->d_sub, d_rout, err,
-                                                              c->stall_tc_mma);
-    DPMM_LAUNCHED();
-    return DPMM_OK;
-}
-
-dpmm_status launch_sub_labels_tc(dpmm_ctx* c, RngArgs r, float* d_rout, bool defer_check)
-{
-    int32_t* err = c->d_aux + 5;
-    DPMM_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int32_t), c->stream));
-    if (c->Dp == 64) DPMM_TRY(launch_sub_labels_tc_t<64>(c, r, d_rout, err));
-    else DPMM_TRY(launch_sub_labels_tc_t<32>(c, r, d_rout, err));
-    if (defer_check) {
-        c->sub_err_pending = true;
-        return DPMM_OK;
-    }
-    int32_t h_err = 0;
-    DPMM_CUDA_TRY(cudaMemcpyAsync(&h_err, err, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-    DPMM_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    if (h_err) return fail(DPMM_ERR_TIMEOUT, "tensor-core sub-label kernel: bounded wait expired (code " +
                                                  std::to_string(h_err) + ")");
     return DPMM_OK;
 }
@@ -2903,7 +2473,7 @@ static int mt_kp(int K) { return std::max(32, (K + 31) / 32 * 32); }
 
 static int mt_stages(int Kp)
 {
-    const size_t avail = kTcSmemCap - 1024 - 256;
+    const size_t avail = tc::kTcSmemCap - 1024 - 256;
     return (int)std::min<size_t>(tc::MT_MAX_STAGES, avail / tc::mt_stage_bytes(Kp));
 }
 
