@@ -252,9 +252,10 @@ extern "C" dpmm_status dpmm_create(const dpmm_desc* desc, dpmm_ctx** out)
     c->nblk_hist = (int)((N + 2047) / 2048);
     {
         // about four waves of two blocks per SM over N points, in whole units, at most kChunkMax
+        const int unit = gauss ? kChunkUnit : kMultChunkUnit;
         const int64_t want = N / ((int64_t)c->num_sms * 2 * 4);
-        const int64_t units = std::max<int64_t>(1, std::min<int64_t>(kChunkMax / kChunkUnit, (want + kChunkUnit - 1) / kChunkUnit));
-        c->chunk_len = (int)(units * kChunkUnit);
+        const int64_t units = std::max<int64_t>(1, std::min<int64_t>(kChunkMax / unit, (want + unit - 1) / unit));
+        c->chunk_len = (int)(units * unit);
     }
     c->max_chunks = (int)(N / c->chunk_len) + KM + 1;
     const int T = Dp * (Dp + 1) / 2;

@@ -23,6 +23,9 @@ constexpr int kMaxMultDim = 4096;
 // kChunkUnit and kChunkMax, the smallest that still gives about four waves of blocks.
 constexpr int kChunkUnit = 1024;
 constexpr int kChunkMax = 4096;
+// Unit of the multinomial contexts: their sums are whole numbers, so the split is free, and a chunk of few
+// long rows is already enough work for a block (20 011 points: 20 -> 157 blocks).
+constexpr int kMultChunkUnit = 128;
 // Pruned label phase: at most kMaxKForPrune clusters; a chunk keeps at most kPrMaxCand other
 // clusters before it is evaluated against every cluster.
 constexpr int kMaxKForPrune = 256;
