@@ -175,7 +175,7 @@ static void free_ctx(dpmm_ctx* c)
     if (c->device >= 0) cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     void* bufs[] = {c->d_x, c->d_gshift, c->d_labels, c->d_sub, c->d_curand, c->d_Wt, c->d_b, c->d_c, c->d_lrw,
-                    c->d_mu, c->d_perm, c->d_blk_hist, c->d_seg, c->d_chunk, c->d_nchunks, c->d_part, c->d_stats,
+                    c->d_mu, c->d_perm, c->d_blk_hist, c->d_seg, c->d_chunk, c->d_nchunks, c->d_cfirst, c->d_part, c->d_stats,
                     c->d_u, c->d_bits, c->d_remap, c->d_aux, c->d_r64, c->d_dbl_scratch, c->d_prior, c->d_lml,
                     c->d_split_hr, c->d_merge_hr, c->d_post_logdet, c->d_mask, c->d_Btc, c->d_Atc, c->d_rbuf,
                     c->d_rpart, c->d_Bsub, c->d_Bsub32, c->d_scr_rec, c->d_scr_vec, c->d_scr_linv, c->d_scr_feat,
@@ -294,6 +294,7 @@ extern "C" dpmm_status dpmm_create(const dpmm_desc* desc, dpmm_ctx** out)
     chk(dev_alloc(&c->d_seg, (size_t)KM + 2));
     chk(dev_alloc(&c->d_chunk, (size_t)3 * c->max_chunks));
     chk(dev_alloc(&c->d_nchunks, (size_t)1));
+    chk(dev_alloc(&c->d_cfirst, (size_t)KM + 1));
     chk(dev_alloc(&c->d_part, (size_t)c->max_chunks * 2 * SL));
     chk(dev_alloc(&c->d_stats, (size_t)3 * KM * c->stat_len));
     chk(dev_alloc(&c->d_stats_tmp, (size_t)3 * KM * c->stat_len));

@@ -158,6 +158,7 @@ struct dpmm_ctx {
     int32_t* d_seg = nullptr;      // [k_max + 1] segment starts
     int32_t* d_chunk = nullptr;    // [max_chunks][3] (cluster, start, len)
     int32_t* d_nchunks = nullptr;
+    int32_t* d_cfirst = nullptr;   // [k_max + 1] first chunk of each cluster, then their number
     int max_chunks = 0;
     int chunk_len = dpmm::kChunkMax;   // points per chunk (see kChunkUnit)
     int perm_K = -1;               // K the permutation was built for (-1: stale)

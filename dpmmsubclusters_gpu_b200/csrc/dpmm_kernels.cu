@@ -953,14 +953,16 @@ __global__ void k_scan_bins(int32_t* __restrict__ blk_hist, int nblk, int K, int
     if (threadIdx.x == 0) total[k] = carry;
 }
 
-// single block: segment starts and the chunk table (cluster, start, len) of <= chunk_len points
+// single block: segment starts, the chunk table (cluster, start, len) of <= chunk_len points and each cluster's first
+// chunk (cfirst[k]; cfirst[K] = their number)
 __global__ void __launch_bounds__(1024) k_segments(const int32_t* __restrict__ total, int K,
                                                    int32_t* __restrict__ seg, int32_t* __restrict__ chunk,
-                                                   int32_t* __restrict__ nchunks, int max_chunks, int chunk_len)
+                                                   int32_t* __restrict__ nchunks, int32_t* __restrict__ cfirst,
+                                                   int max_chunks, int chunk_len)
 {
     // thread i takes bins [k0, k1); a block scan of the bins' point and chunk totals gives its offsets
-    __shared__ int32_t s_t[1024], s_c[1024];
-    const int tid = threadIdx.x, nthr = blockDim.x;
+    __shared__ int32_t w_t[32], w_c[32], s_first[1025];
+    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const int items = K + 1;   // cluster bins 0..K-1 and bin K (labels outside 1..K: no chunks)
     const int per = (items + nthr - 1) / nthr;
     const int k0 = min(items, tid * per), k1 = min(items, k0 + per);
@@ -970,32 +972,59 @@ __global__ void __launch_bounds__(1024) k_segments(const int32_t* __restrict__ t
         st += t;
         if (k < K) sc += (t + chunk_len - 1) / chunk_len;
     }
-    s_t[tid] = st;
-    s_c[tid] = sc;
-    __syncthreads();
-    for (int o = 1; o < nthr; o <<= 1) {   // inclusive scan
-        const int32_t a = tid >= o ? s_t[tid - o] : 0, c = tid >= o ? s_c[tid - o] : 0;
-        __syncthreads();
-        s_t[tid] += a;
-        s_c[tid] += c;
-        __syncthreads();
+    int32_t it = st, ic = sc;   // inclusive scans
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int32_t a = __shfl_up_sync(0xffffffffu, it, o), c = __shfl_up_sync(0xffffffffu, ic, o);
+        if (lane >= o) {
+            it += a;
+            ic += c;
+        }
     }
-    int32_t acc = s_t[tid] - st, nc = s_c[tid] - sc;
+    if (lane == 31) {
+        w_t[warp] = it;
+        w_c[warp] = ic;
+    }
+    __syncthreads();
+    int32_t bt = 0, bc = 0, all_c = 0;
+    for (int v = 0; v < 32; ++v) {
+        if (v < warp) {
+            bt += w_t[v];
+            bc += w_c[v];
+        }
+        all_c += w_c[v];
+    }
+    it += bt;
+    ic += bc;
+    const int ncall = min(all_c, max_chunks);
+    int32_t acc = it - st, nc = ic - sc;
     for (int k = k0; k < k1; ++k) {
         seg[k] = acc;
         const int32_t t = total[k];
-        if (k < K)
-            for (int32_t s = 0; s < t; s += chunk_len, ++nc)
-                if (nc < max_chunks) {
-                    chunk[3 * nc + 0] = k;
-                    chunk[3 * nc + 1] = acc + s;
-                    chunk[3 * nc + 2] = min(chunk_len, t - s);
-                }
+        if (k < K) cfirst[k] = min(nc, ncall);
+        if (per == 1 && k < K) s_first[k] = nc;
+        if (k < K) nc += (t + chunk_len - 1) / chunk_len;
         acc += t;
     }
     if (tid == nthr - 1) {
-        seg[K + 1] = s_t[nthr - 1];
-        *nchunks = min(s_c[nthr - 1], max_chunks);
+        seg[K + 1] = it;
+        *nchunks = ncall;
+        cfirst[K] = ncall;
+    }
+    __syncthreads();
+    // the chunk table, a chunk per thread (a serial loop per cluster took 50 stores in a row at 50 chunks): the
+    // cluster is the last one whose first chunk is not past it
+    for (int q = tid; q < ncall; q += nthr) {
+        int lo = 0, hi = K - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) / 2;
+            if ((per == 1 ? s_first[mid] : cfirst[mid]) <= q) lo = mid;
+            else hi = mid - 1;
+        }
+        const int32_t s = (q - (per == 1 ? s_first[lo] : cfirst[lo])) * chunk_len;
+        chunk[3 * q + 0] = lo;
+        chunk[3 * q + 1] = seg[lo] + s;
+        chunk[3 * q + 2] = min(chunk_len, total[lo] - s);
     }
 }
 
@@ -1040,8 +1069,8 @@ dpmm_status build_permutation(dpmm_ctx* c, int K)
     int32_t* total = c->d_aux + 8;   // K+1 entries
     k_scan_bins<<<K + 1, 1024, 0, c->stream>>>(c->d_blk_hist, nblk, K, total);
     DPMM_LAUNCHED();
-    k_segments<<<1, 1024, 0, c->stream>>>(total, K, c->d_seg, c->d_chunk, c->d_nchunks, c->max_chunks,
-                                         c->chunk_len);
+    k_segments<<<1, 1024, 0, c->stream>>>(total, K, c->d_seg, c->d_chunk, c->d_nchunks, c->d_cfirst,
+                                         c->max_chunks, c->chunk_len);
     DPMM_LAUNCHED();
     size_t sm = sizeof(int32_t) * 9 * (K + 1);
     if (sm > 48 * 1024) DPMM_CUDA_TRY(cudaFuncSetAttribute(k_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -1680,6 +1709,19 @@ __global__ void __launch_bounds__(256) k_mult_sub_stats(
                 const float4* src = reinterpret_cast<const float4*>(x + (size_t)sperm[t % 3][row] * Dp) + c;
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * (uint32_t)e), "l"(src) : "memory");
             }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (tid < R) {
+        sperm[0][tid] = perm_of(0);
+        sperm[1][tid] = perm_of(1);
+    }
+    __syncthreads();
+    stage_rows(0);
+    stage_rows(1);
+    // sums: this thread's categories 4 (c + 256 q) .. + 3 of the points g, g + G, ..
+    const int G = C4 < 256 ? 256 / C4 : 1, g = C4 < 256 ? tid / C4 : 0, c = C4 < 256 ? tid % C4 : tid;
+    float4 al[NG], ar[NG];
 #pragma unroll
     for (int q = 0; q < NG; ++q) al[q] = ar[q] = make_float4(0.f, 0.f, 0.f, 0.f);
     int cnt_l = 0, cnt_r = 0;
@@ -1738,6 +1780,8 @@ __global__ void __launch_bounds__(256) k_mult_sub_stats(
                 draw_uniform2(rng, pt, u1, u2);
                 sv = draw_sub_label(dl + wl, dr + wr, u1, u2);
                 sub[pt] = sv;
+            } else {
+                sv = sub[pt];
             }
             ssub[tid] = sv;
         }
@@ -1765,7 +1809,11 @@ __global__ void __launch_bounds__(256) k_mult_sub_stats(
                 }
             }
         }
+        if (tid < R) sperm[(t + 2) % 3][tid] = next;
+        __syncthreads();   // the rows are read, the entries of tile t + 2 written
+        stage_rows(t + 2);
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     double* pl = part + (size_t)ch * 2 * SL;
     double* pr = pl + SL;
@@ -1815,19 +1863,6 @@ static dpmm_status launch_mult_sub_stats_t(dpmm_ctx* c, RngArgs r, float* d_rout
     DPMM_LAUNCHED();
     return DPMM_OK;
 }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    if (tid < R) {
-        sperm[0][tid] = perm_of(0);
-        sperm[1][tid] = perm_of(1);
-    }
-    __syncthreads();
-    stage_rows(0);
-    stage_rows(1);
-    // sums: this thread's categories 4 (c + 256 q) .. + 3 of the points g, g + G, ..
-    const int G = C4 < 256 ? 256 / C4 : 1, g = C4 < 256 ? tid / C4 : 0, c = C4 < 256 ? tid % C4 : tid;
-    float4 al[NG], ar[NG];
 
 template <int DP>
 static dpmm_status launch_gauss_sub_stats_t(dpmm_ctx* c, int draw, RngArgs r, float* d_rout, const uint8_t* d_mask)
@@ -1840,8 +1875,6 @@ static dpmm_status launch_gauss_sub_stats_t(dpmm_ctx* c, int draw, RngArgs r, fl
             DPMM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
             KernelTimer kt(d_mask ? nullptr : c, PH_SLOT_STATS);   // full launches only (masked: a few clusters)
             kern<<<c->max_chunks, 256, sm, c->stream>>>(c->d_x, c->d_perm, c->d_chunk, c->d_nchunks, c->d_mu,
-            } else {
-                sv = sub[pt];
                                                         c->d_sub, c->d_part, d_mask);
             DPMM_LAUNCHED();
             return DPMM_OK;
@@ -1852,11 +1885,7 @@ static dpmm_status launch_gauss_sub_stats_t(dpmm_ctx* c, int draw, RngArgs r, fl
     DPMM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     kern<<<c->max_chunks, 256, sm, c->stream>>>(c->d_x, c->d_perm, c->d_chunk, c->d_nchunks, c->d_Wt, c->d_b, c->d_c,
                                                 c->d_lrw, c->d_mu, draw, r, c->d_sub, d_rout, c->d_part, d_mask);
-        if (tid < R) sperm[(t + 2) % 3][tid] = next;
-        __syncthreads();   // the rows are read, the entries of tile t + 2 written
-        stage_rows(t + 2);
     DPMM_LAUNCHED();
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
     return DPMM_OK;
 }
 
@@ -1896,44 +1925,77 @@ dpmm_status launch_sub_labels_and_stats(dpmm_ctx* c, int K, const float* d_u, fl
     return launch_stats_finalize(c, K, d_mask);
 }
 
-// Blocks (cluster, share of the scatter triangle): chunk partials summed in chunk order (FP64),
-// shifted back to the original coordinates, written as count / sum / full S for slots 3k
-// (cluster = l + r), 3k+1 (l), 3k+2 (r).
-__global__ void k_stats_finalize(const double* __restrict__ part, const int32_t* __restrict__ chunk,
-                                 const int32_t* __restrict__ nchunks, const float* __restrict__ muv,
+// sums over the chunks [c0, c1) of one value of their two records (l, r), in chunk order; 16 loads ahead of the
+// additions (a chunk's load used to wait for the addition before it)
+__device__ __forceinline__ double2 sum_chunks(const double* __restrict__ p, size_t SL, int c0, int c1)
+{
+    double2 acc = make_double2(0.0, 0.0);
+    for (int q = c0; q < c1; q += 8) {
+        double l[8], r[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const double* at = p + (size_t)(q + u) * 2 * SL;
+            l[u] = q + u < c1 ? at[0] : 0.0;
+            r[u] = q + u < c1 ? at[SL] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            acc.x += l[u];
+            acc.y += r[u];
+        }
+    }
+    return acc;
+}
+
+// Blocks (cluster, share of its values): chunk partials summed in chunk order (FP64), shifted back to the original
+// coordinates, written as count / sum / full S for slots 3k (cluster = l + r), 3k+1 (l), 3k+2 (r).  The shares
+// divide the upper triangle (Gaussian; every share sums the counts and sums it needs) or the counts
+// (multinomial).  Bound by the latency of the chunks' records: the first chunks come from k_segments, the loads
+// run ahead, and a share's triangle sums start before its counts are waited for (K = 20, D = 32, 1000 chunks:
+// 50 -> 16 us; K = 2, D = 2, 98 chunks: 34 -> 10 us; multinomial, K = 50, D = 1000, 800 chunks: 51 -> 8 us).
+__global__ void __launch_bounds__(256) k_stats_finalize(const double* __restrict__ part, const int32_t* __restrict__ cfirst,
+                                 const float* __restrict__ muv,
                                  const double* __restrict__ gshift, int D, int Dp, int gauss, int SL, int out_len,
                                  double* __restrict__ stats, const uint8_t* __restrict__ mask)
 {
     const int k = blockIdx.x;
     if (mask && !mask[k]) return;
-    const int nc = *nchunks;
-    // first chunk of this cluster (chunks are ordered by cluster)
-    int lo = 0, hi = nc;
-    while (lo < hi) {
-        int mid = (lo + hi) / 2;
-        if (chunk[3 * mid] < k) lo = mid + 1; else hi = mid;
-    }
-    const int c0 = lo;
-    int c1 = c0;
-    while (c1 < nc && chunk[3 * c1] == k) ++c1;
-    const int T = gauss ? Dp * (Dp + 1) / 2 : 0;
-    extern __shared__ double shd[];
-    double* n2 = shd;                 // [2]
-    double* sm2 = shd + 2;            // [2][D]
-    double* t = sm2 + 2 * D;          // [D] total shift (gauss)
-    for (int s = 0; s < 2; ++s) {
-        for (int e = threadIdx.x; e < 1 + D; e += blockDim.x) {
-            double acc = 0.0;
-            for (int q = c0; q < c1; ++q) acc += part[((size_t)q * 2 + s) * SL + e];
-            if (e == 0) n2[s] = acc; else sm2[s * D + e - 1] = acc;
-        }
-    }
-    if (gauss)
-        for (int e = threadIdx.x; e < D; e += blockDim.x) t[e] = (double)muv[(size_t)3 * k * Dp + e] + gshift[e];
-    __syncthreads();
+    const int c0 = cfirst[k], c1 = cfirst[k + 1];   // chunks are ordered by cluster
     double* out_c = stats + (size_t)(3 * k) * out_len;
     double* out_l = out_c + out_len;
     double* out_r = out_l + out_len;
+    if (!gauss) {
+        for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < 1 + D; e += gridDim.y * blockDim.x) {
+            const double2 v = sum_chunks(part + e, (size_t)SL, c0, c1);
+            out_l[e] = v.x;
+            out_r[e] = v.y;
+            out_c[e] = v.x + v.y;
+        }
+        return;
+    }
+    const int T = Dp * (Dp + 1) / 2;
+    extern __shared__ double shd[];
+    double* n2 = shd;                 // [2]
+    double* sm2 = shd + 2;            // [2][D]
+    double* t = sm2 + 2 * D;          // [D] total shift
+    // S = Sc + t Sc_sum^T + Sc_sum t^T + n t t^T, with Sc_sum = sum (x - t); block y of the cluster takes the
+    // y-th share of the upper triangle
+    const int per = (T + (int)gridDim.y - 1) / (int)gridDim.y;
+    const int e0 = per * (int)blockIdx.y + threadIdx.x, e1 = min(T, per * ((int)blockIdx.y + 1));
+    double2 first = make_double2(0.0, 0.0);
+    if (e0 < e1) first = sum_chunks(part + 1 + Dp + e0, (size_t)SL, c0, c1);
+    for (int e = (int)blockDim.x - 1 - (int)threadIdx.x; e < 1 + D; e += blockDim.x) {
+        const double2 v = sum_chunks(part + e, (size_t)SL, c0, c1);
+        if (e == 0) {
+            n2[0] = v.x;
+            n2[1] = v.y;
+        } else {
+            sm2[e - 1] = v.x;
+            sm2[D + e - 1] = v.y;
+        }
+    }
+    for (int e = threadIdx.x; e < D; e += blockDim.x) t[e] = (double)muv[(size_t)3 * k * Dp + e] + gshift[e];
+    __syncthreads();
     if (blockIdx.y == 0) {
         if (threadIdx.x == 0) {
             out_l[0] = n2[0];
@@ -1942,26 +2004,25 @@ __global__ void k_stats_finalize(const double* __restrict__ part, const int32_t*
         }
         for (int e = threadIdx.x; e < D; e += blockDim.x) {
             double sl = sm2[e], sr = sm2[D + e];
-            if (gauss) { sl += n2[0] * t[e]; sr += n2[1] * t[e]; }
+            sl += n2[0] * t[e];
+            sr += n2[1] * t[e];
             out_l[1 + e] = sl;
             out_r[1 + e] = sr;
             out_c[1 + e] = sl + sr;
         }
     }
-    if (!gauss) return;
-    // S = Sc + t Sc_sum^T + Sc_sum t^T + n t t^T, with Sc_sum = sum (x - t); block y of the
-    // cluster takes the y-th share of the upper triangle
-    const int per = (T + (int)gridDim.y - 1) / (int)gridDim.y;
-    const int e1 = min(T, per * ((int)blockIdx.y + 1));
-    for (int e = per * (int)blockIdx.y + threadIdx.x; e < e1; e += blockDim.x) {
-        int i = 0, rem = e;
-        while (rem >= Dp - i) { rem -= Dp - i; ++i; }
-        int j = i + rem;
+    for (int e = e0; e < e1; e += blockDim.x) {
+        const double2 sc = e == e0 ? first : sum_chunks(part + 1 + Dp + e, (size_t)SL, c0, c1);
+        // row i of the triangle starts at i (2 Dp + 1 - i) / 2
+        const float b2 = (float)(2 * Dp + 1);
+        int i = (int)((b2 - sqrtf(b2 * b2 - 8.f * (float)e)) * 0.5f);
+        if (i * (2 * Dp + 1 - i) / 2 > e) --i;
+        else if ((i + 1) * (2 * Dp - i) / 2 <= e) ++i;
+        const int j = i + e - i * (2 * Dp + 1 - i) / 2;
         if (i >= D || j >= D) continue;
         double v[2];
         for (int s = 0; s < 2; ++s) {
-            double acc = 0.0;
-            for (int q = c0; q < c1; ++q) acc += part[((size_t)q * 2 + s) * SL + 1 + Dp + e];
+            const double acc = s ? sc.y : sc.x;
             double si = sm2[s * D + i], sj = sm2[s * D + j];
             v[s] = acc + t[i] * sj + si * t[j] + n2[s] * t[i] * t[j];
         }
@@ -1994,8 +2055,10 @@ dpmm_status launch_stats_finalize(dpmm_ctx* c, int K, const uint8_t* d_mask)
     size_t sm = sizeof(double) * (2 + 3 * (size_t)c->D);
     if (sm > 48 * 1024)
         DPMM_CUDA_TRY(cudaFuncSetAttribute(k_stats_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    const dim3 grid((unsigned)K, gauss ? 8u : 1u);   // the scatter triangle over 8 blocks per cluster
-    k_stats_finalize<<<grid, 256, sm, c->stream>>>(c->d_part, c->d_chunk, c->d_nchunks, c->d_mu, c->d_gshift, c->D,
+    // a block's worth of values per share where K leaves room on the device
+    const int values = gauss ? tri(c->Dp) : 1 + c->D;
+    const dim3 grid((unsigned)K, (unsigned)std::max(1, std::min((values + 255) / 256, gauss ? 8 : 16)));
+    k_stats_finalize<<<grid, 256, sm, c->stream>>>(c->d_part, c->d_cfirst, c->d_mu, c->d_gshift, c->D,
                                                 c->Dp, gauss, SL, c->stat_len, c->d_stats, d_mask);
     DPMM_LAUNCHED();
     if (c->shard_world > 1) {
