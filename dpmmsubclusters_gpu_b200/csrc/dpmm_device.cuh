@@ -210,27 +210,42 @@ __device__ __forceinline__ int draw_sub_label(float rl, float rr, float u1, floa
 //    when D > C, is aliased to the next large with positive excess.
 // The merge stops as soon as the drawn column is settled.  D and C are FP64 running sums in the
 // reference's consumption order.
-// Small/large flags of up to 256 categories as a bitmask in registers: bit (q - 1) % 32 of word
-// (q - 1) / 32 is set when category q is small.  The walks of the merge become bit scans.
+// Small/large flags of up to 32 NW categories as a bitmask in registers: bit (q - 1) % 32 of word
+// (q - 1) / 32 is set when category q is small.  The walks of the merge become bit scans, whose cost grows
+// with the words, so the draw takes the fewest that hold K.
+template <int NW>
 struct SmallMask {
-    uint32_t w[8];
+    uint32_t w[NW];
+    uint32_t below[NW];   // y < 1 not ruled out (the flag itself may come from another test than y < 1)
     int K;
 
     __device__ __forceinline__ uint32_t word(int i) const
     {
-        uint32_t v = 0;
+        uint32_t v = w[0];
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
+        for (int j = 1; j < NW; ++j)
             if (j == i) v = w[j];
         return v;
     }
     __device__ __forceinline__ bool small(int q) const { return (word((q - 1) >> 5) >> ((q - 1) & 31)) & 1u; }
+    // y < 1 is ruled out for none of the categories q .. q + 7
+    __device__ __forceinline__ bool below8(int q) const
+    {
+        const int i = (q - 1) >> 5;
+        uint32_t lo = below[0], hi = 0u;
+#pragma unroll
+        for (int j = 1; j < NW; ++j) {
+            if (j == i) lo = below[j];
+            if (j == i + 1) hi = below[j];
+        }
+        return (__funnelshift_r(lo, hi, (q - 1) & 31) & 0xffu) == 0xffu;
+    }
     // smallest small q > x (K + 1 if none)
     __device__ __forceinline__ int next_small_after(int x) const
     {
         int res = K + 1;
 #pragma unroll
-        for (int j = 7; j >= 0; --j) {
+        for (int j = NW - 1; j >= 0; --j) {
             uint32_t m = w[j];
             const int lo = x - 32 * j;   // clear bits b with 32j + b + 1 <= x
             m = lo <= 0 ? m : (lo >= 32 ? 0u : m & (~0u << lo));
@@ -243,7 +258,7 @@ struct SmallMask {
     {
         int res = 0;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < NW; ++j) {
             const int nv = K - 32 * j;   // valid bits in word j
             uint32_t m = ~w[j] & (nv >= 32 ? ~0u : (nv <= 0 ? 0u : (1u << nv) - 1u));
             const int hi = x - 1 - 32 * j;   // keep bits b with 32j + b + 1 < x
@@ -260,6 +275,7 @@ struct ReadFlags {
     YF y;
     int K;
     __device__ __forceinline__ bool small(int q) const { return y(q - 1) < 1.f; }
+    __device__ __forceinline__ bool below8(int) const { return true; }   // (the values are looked at anyway)
     __device__ __forceinline__ int next_small_after(int x) const
     {
         int q = x + 1;
@@ -319,8 +335,9 @@ __device__ __forceinline__ int alias_merge(const YF& y, int K, int ns, const Fla
         // Fast path: the next 8 positions of the small stream hold their own smalls (no displaced
         // large among them), col is not one of them, and the current large still has capacity
         // after all 8: none of these steps can change the outcome, so take them at once (same
-        // summation order as single steps).
-        if (cur != 0 && P > 8 && (col >= P || col < P - 8)) {
+        // summation order as single steps).  The attempt is left out where one of them is clearly large:
+        // eight exponentials at every step cost more than the merge.
+        if (cur != 0 && P > 8 && (col >= P || col < P - 8) && fl.below8(P - 8)) {
             float v[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = y(P - 2 - i);
@@ -360,37 +377,49 @@ __device__ __forceinline__ int alias_merge(const YF& y, int K, int ns, const Fla
     }
 }
 
-// Alias draw over K categories given y(i) = p_{i+1} * K (FP32): register bitmask walks for
-// K <= 256, reads otherwise.  SF: is_small(i), the small/large split the merge follows (y(i) < 1,
-// or an equivalent cheaper test; at an exact tie either answer keeps the walk consistent: a
-// small with y >= 1 adds no deficit and a large with y <= 1 has no excess to give).
-template <typename YF, typename SF>
-__device__ __forceinline__ int alias_draw_y(const YF& y, const SF& is_small, int K, float u1, float u2)
+// Alias draw over K <= 32 NW categories given y(i) = p_{i+1} * K (FP32) with register bitmask walks.
+// SF: flags(i), bit 0 the small/large split the merge follows (y(i) < 1, or an equivalent cheaper test; at an
+// exact tie either answer keeps the walk consistent: a small with y >= 1 adds no deficit and a large with
+// y <= 1 has no excess to give), bit 1 set wherever y(i) < 1; called once per i, in order.
+template <int NW, typename YF, typename SF>
+__device__ __forceinline__ int alias_draw_mask(const YF& y, const SF& flags, int K, float u1, float u2)
 {
-    if (K <= 256) {
-        SmallMask sm;
-        sm.K = K;
-        int ns = 0;
+    SmallMask<NW> sm;
+    sm.K = K;
+    int ns = 0;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            uint32_t m = 0;
-            const int kend = min(K, 32 * j + 32);
-            for (int k = 32 * j; k < kend; ++k) m |= (is_small(k) ? 1u : 0u) << (k - 32 * j);
-            sm.w[j] = m;
-            ns += __popc(m);
+    for (int j = 0; j < NW; ++j) {
+        uint32_t m = 0, b = 0;
+        const int kend = min(K, 32 * j + 32);
+#pragma unroll 8
+        for (int k = 32 * j; k < kend; ++k) {
+            const uint32_t f = flags(k);
+            m |= (f & 1u) << (k - 32 * j);
+            b |= (f >> 1) << (k - 32 * j);
         }
-        if (ns == K - 1) {
-            // One large L: it absorbs every small's deficit (its excess equals their total up to
-            // rounding, well below 1e-3), so a drawn small with y < 0.999 is aliased to L wherever it
-            // sits in the consumption order.  Otherwise (col = L, or y near 1) walk the merge.
-            const int col = alias_column(K, u1);
-            if (sm.small(col)) {
-                const float yc = y(col - 1);
-                if (yc < 0.999f) return yc < u2 ? sm.prev_large_before(K + 1) : col;
-            }
-        }
-        return alias_merge(y, K, ns, sm, u1, u2);
+        sm.w[j] = m;
+        sm.below[j] = b;
+        ns += __popc(m);
     }
+    if (ns == K - 1) {
+        // One large L: it absorbs every small's deficit (its excess equals their total up to
+        // rounding, well below 1e-3), so a drawn small with y < 0.999 is aliased to L wherever it
+        // sits in the consumption order.  Otherwise (col = L, or y near 1) walk the merge.
+        const int col = alias_column(K, u1);
+        if (sm.small(col)) {
+            const float yc = y(col - 1);
+            if (yc < 0.999f) return yc < u2 ? sm.prev_large_before(K + 1) : col;
+        }
+    }
+    return alias_merge(y, K, ns, sm, u1, u2);
+}
+
+// The same for any K: reads instead of the bitmask above 256.
+template <typename YF, typename SF>
+__device__ __forceinline__ int alias_draw_y(const YF& y, const SF& flags, int K, float u1, float u2)
+{
+    if (K <= 32) return alias_draw_mask<1>(y, flags, K, u1, u2);
+    if (K <= 256) return alias_draw_mask<8>(y, flags, K, u1, u2);
     int ns = 0;
     for (int k = 0; k < K; ++k) ns += y(k) < 1.f ? 1 : 0;
     return alias_merge(y, K, ns, ReadFlags<YF>{y, K}, u1, u2);
@@ -401,8 +430,8 @@ __device__ __forceinline__ int alias_draw_stream(const float* __restrict__ ys, i
                                                  float u2)
 {
     auto y = [=](int i) -> float { return ys[(size_t)i * stride]; };
-    auto is_small = [=](int i) -> bool { return ys[(size_t)i * stride] < 1.f; };
-    return alias_draw_y(y, is_small, K, u1, u2);
+    auto flags = [=](int i) -> uint32_t { return ys[(size_t)i * stride] < 1.f ? 3u : 0u; };
+    return alias_draw_y(y, flags, K, u1, u2);
 }
 
 }  // namespace dpmm

@@ -426,10 +426,18 @@ __global__ void __launch_bounds__(THREADS, 1) k_gauss_labels_tc(
 // Softmax + alias draw (or argmax) per point from the label kernel's r (cluster-major) and the
 // two halves' partials: build_log_likelihood_array_kernel + sample_by_probability
 // (cudaKernel.cu:374-403, 27-124) or update_labels_by_max_index_kernel (:405-424).
+//
+// NW: words of the small/large mask (K <= 32 NW); NW = 0: any K.  STAGED: the point's r are kept in shared memory
+// as the mask is built (K x 256 floats), because the merge of a point with several large clusters reads
+// them again in an order of its own, one dependent load after the other.  Bound: that merge where the clusters
+// overlap (K = 20, 1e6 points: 194 -> 95 us; K = 64, 3e5 points: 191 -> 122 us, of which reading r takes 12), the
+// reads of r where they do not.
+template <int NW, bool STAGED>
 __global__ void __launch_bounds__(256) k_draw_labels(const float* __restrict__ rbuf, const float* __restrict__ part,
                                                      int64_t N, int K, int final_, RngArgs rng,
                                                      int32_t* __restrict__ labels)
 {
+    extern __shared__ float sr[];   // [K][256] (STAGED)
     const int64_t pt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (pt >= N) return;
     const float m0 = part[pt], x0 = part[N + pt], m1 = part[2 * N + pt], x1 = part[3 * N + pt];
@@ -445,13 +453,53 @@ __global__ void __launch_bounds__(256) k_draw_labels(const float* __restrict__ r
     const float sum = x0 * __expf(m0 - mx) + x1 * __expf(m1 - mx);
     const float inv = 1.0f / sum, fk = (float)K;
     const float* rp = rbuf + pt;
-    auto y = [=](int i) -> float { return (__expf(__ldg(rp + (size_t)i * N) - mx) * inv) * fk; };
     // y < 1  <=>  r < max + log(sum / K): one compare per cluster for the small/large split
     const float thr = mx + __logf(sum / fk);
-    auto is_small = [=](int i) -> bool { return __ldg(rp + (size_t)i * N) < thr; };
+    // ... up to the rounding of either: wherever y < 1, r is below this
+    const float thr_hi = thr + 1e-3f + 1e-6f * fabsf(thr);
     float u1, u2;
     draw_uniform2(rng, pt, u1, u2);
-    labels[pt] = alias_draw_y(y, is_small, K, u1, u2);
+    if constexpr (STAGED) {
+        float* own = sr + threadIdx.x;
+        auto y = [=](int i) -> float { return (__expf(own[256 * i] - mx) * inv) * fk; };
+        auto flags = [=](int i) -> uint32_t {
+            const float r = __ldg(rp + (size_t)i * N);
+            own[256 * i] = r;
+            return (r < thr ? 1u : 0u) | (r < thr_hi ? 2u : 0u);
+        };
+        labels[pt] = alias_draw_mask<NW>(y, flags, K, u1, u2);
+    } else {
+        auto y = [=](int i) -> float { return (__expf(__ldg(rp + (size_t)i * N) - mx) * inv) * fk; };
+        auto flags = [=](int i) -> uint32_t {
+            const float r = __ldg(rp + (size_t)i * N);
+            return (r < thr ? 1u : 0u) | (r < thr_hi ? 2u : 0u);
+        };
+        if constexpr (NW == 0) labels[pt] = alias_draw_y(y, flags, K, u1, u2);
+        else labels[pt] = alias_draw_mask<NW>(y, flags, K, u1, u2);
+    }
+}
+
+template <int NW, bool STAGED>
+static dpmm_status launch_draw_labels_t(dpmm_ctx* c, int K, int final_, const RngArgs& r)
+{
+    const size_t sm = STAGED && !final_ ? sizeof(float) * 256 * (size_t)K : 0;
+    if (sm > 48 * 1024)
+        DPMM_CUDA_TRY(cudaFuncSetAttribute(k_draw_labels<NW, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    k_draw_labels<NW, STAGED><<<(unsigned)((c->N + 255) / 256), 256, sm, c->stream>>>(c->d_rbuf, c->d_rpart, c->N, K, final_, r,
+                                                                                    c->d_labels);
+    DPMM_LAUNCHED();
+    return DPMM_OK;
+}
+
+// staged up to the K whose columns leave two blocks per SM (96 KB each)
+static dpmm_status launch_draw_labels(dpmm_ctx* c, int K, int final_, const RngArgs& r)
+{
+    if (K <= 32) return launch_draw_labels_t<1, true>(c, K, final_, r);
+    if (K <= 64) return launch_draw_labels_t<2, true>(c, K, final_, r);
+    if (K <= 96) return launch_draw_labels_t<3, true>(c, K, final_, r);
+    if (K <= 128) return launch_draw_labels_t<4, false>(c, K, final_, r);
+    if (K <= 256) return launch_draw_labels_t<8, false>(c, K, final_, r);
+    return launch_draw_labels_t<0, false>(c, K, final_, r);
 }
 
 // ------------------------------------------------------------------------- pruned-phase scan
@@ -2084,9 +2132,7 @@ dpmm_status launch_cluster_labels_tc(dpmm_ctx* c, int K, int final_, const float
         DPMM_LAUNCHED();
     }
     RngArgs r = rng_args(c, d_u);
-    tc::k_draw_labels<<<(unsigned)((c->N + 255) / 256), 256, 0, c->stream>>>(c->d_rbuf, c->d_rpart, c->N, K, final_,
-                                                                            r, c->d_labels);
-    DPMM_LAUNCHED();
+    DPMM_TRY(tc::launch_draw_labels(c, K, final_, r));
     int32_t h_err = 0;
     DPMM_CUDA_TRY(cudaMemcpyAsync(&h_err, err, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
     DPMM_CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -2543,9 +2589,7 @@ dpmm_status launch_mult_labels_tc(dpmm_ctx* c, int K, int final_, const float* d
         DPMM_LAUNCHED();
     }
     RngArgs r = rng_args(c, d_u);
-    tc::k_draw_labels<<<(unsigned)((c->N + 255) / 256), 256, 0, c->stream>>>(c->d_rbuf, c->d_rpart, c->N, K, final_,
-                                                                            r, c->d_labels);
-    DPMM_LAUNCHED();
+    DPMM_TRY(tc::launch_draw_labels(c, K, final_, r));
     int32_t h_err = 0;
     DPMM_CUDA_TRY(cudaMemcpyAsync(&h_err, err, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
     DPMM_CUDA_TRY(cudaStreamSynchronize(c->stream));
