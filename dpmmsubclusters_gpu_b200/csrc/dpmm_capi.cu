@@ -178,7 +178,7 @@ static void free_ctx(dpmm_ctx* c)
                     c->d_mu, c->d_perm, c->d_blk_hist, c->d_seg, c->d_chunk, c->d_nchunks, c->d_cfirst, c->d_part, c->d_stats,
                     c->d_u, c->d_bits, c->d_remap, c->d_aux, c->d_r64, c->d_dbl_scratch, c->d_prior, c->d_lml,
                     c->d_split_hr, c->d_merge_hr, c->d_post_logdet, c->d_mask, c->d_Btc, c->d_Atc, c->d_rbuf,
-                    c->d_rpart, c->d_Bsub, c->d_Bsub32, c->d_scr_rec, c->d_scr_vec, c->d_scr_linv, c->d_scr_feat,
+                    c->d_rpart, c->d_Bsub, c->d_Bsub32, c->d_Blab32, c->d_scr_rec, c->d_scr_vec, c->d_scr_linv, c->d_scr_feat,
                     c->d_scr_prox, c->d_scr_score, c->d_scr_w, c->d_scr_wdep, c->d_scr_elig, c->d_scr_sel,
                     c->d_scr_list, c->d_scr_slots, c->d_scr_hr, c->d_stats_tmp, c->d_logw, c->d_prune_rh,
                     c->d_prune_cand, c->d_prune_lam, c->d_prune_M, c->d_prune_cnt, c->d_prune_V,
@@ -274,7 +274,8 @@ extern "C" dpmm_status dpmm_create(const dpmm_desc* desc, dpmm_ctx** out)
         chk(dev_alloc(&c->d_b, (size_t)3 * KM * Dp));
         if ((Dp == 32 || Dp == 64) && c->ll_mode != DPMM_LL_FP32) {
             chk(dev_alloc(&c->d_Btc, tc_param_bytes(KM)));
-            chk(dev_alloc(&c->d_Atc, (size_t)((N + 127) / 128) * 32768));
+            chk(dev_alloc(&c->d_Atc, tc_point_bytes(N, Dp)));
+            if (Dp == 32) chk(dev_alloc(&c->d_Blab32, tc_param32_bytes(KM)));
             chk(dev_alloc(&c->d_rbuf, (size_t)N * KM));
             chk(dev_alloc(&c->d_rpart, (size_t)4 * N));
             chk(dev_alloc(&c->d_Bsub, (size_t)KM * 32768));

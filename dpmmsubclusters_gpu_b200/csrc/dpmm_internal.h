@@ -136,8 +136,10 @@ struct dpmm_ctx {
     float* d_mu = nullptr;         // [3*k_max][Dp], mu - shift (Gaussian) / log theta (multinomial)
     uint8_t* d_Btc = nullptr;      // tensor-core B operand: per pair of clusters a 32 KB split-bf16,
                                    // K-major 128-byte-swizzled tile (Gaussian, Dp = 32 or 64)
-    uint8_t* d_Atc = nullptr;      // tensor-core A operand: per 128 points the same 32 KB split-bf16
-                                   // swizzled tile, packed once when the points are uploaded
+    uint8_t* d_Atc = nullptr;      // tensor-core A operand: per 128 points one split-bf16 swizzled tile (32 KB; Dp = 32:
+                                   // 16 KB of rows [32 hi | 32 lo]), packed once when the points are uploaded
+    uint8_t* d_Blab32 = nullptr;   // dense label kernel's B operand at Dp = 32: per four clusters 16 KB, then the
+                                   // bias records (the pruned phase's scans read d_Btc)
     uint8_t* d_Bsub = nullptr;     // tensor-core sub-label phase: per cluster its two sub-cluster
                                    // factors as one 32 KB split-bf16 swizzled B tile (Dp = 32: the fused
                                    // sub-label + statistics pass only, packed while it is on)
@@ -370,6 +372,8 @@ dpmm_status pack_mult_tc_points(dpmm_ctx* c);          // the counts as BF16 til
 dpmm_status pack_mult_tc_params(dpmm_ctx* c, int K);   // log theta as three BF16 parts
 dpmm_status launch_mult_labels_tc(dpmm_ctx* c, int K, int final_, const float* d_u, float* d_rout);
 size_t tc_param_bytes(int k_max);          // B tiles + bias records for k_max clusters
+size_t tc_param32_bytes(int k_max);        // the same for the half-width operands of Dp = 32
+size_t tc_point_bytes(int64_t N, int Dp);  // A operand of N points
 // tensor-core sub-label kernel (dpmm_rows_tc.cu): draws the sub-labels only (statistics separately)
 bool tc_sub_supported(const dpmm_ctx* c);
 // defer_check: its error word is read by the statistics launch that follows (one sync for both)

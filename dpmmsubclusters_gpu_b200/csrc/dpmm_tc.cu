@@ -34,12 +34,11 @@ constexpr int BN = CPT * KD;               // 128 accumulator columns per N tile
 constexpr int B_BYTES = BN * KD * 2;       // 16 KB (one of hi / lo)
 constexpr int STAGE_BYTES = 2 * B_BYTES;   // 32 KB: hi then lo
 constexpr uint32_t TMEM_COLS = 512;        // 2 accumulator pairs: 2 halves x 128 columns each
+constexpr int LABEL_PASS = 256;            // clusters per launch: their biases stay in shared memory (67 KB at D = 64)
 constexpr int NPAIR = 2;                   // accumulator pairs (N tiles in flight)
 constexpr int HALVES = 2;                  // point tiles per super-tile (M = 2 x 128 per B tile)
-constexpr int A_SLOT = HALVES * 2 * A_BYTES;   // 64 KB: tile 0 hi, lo, tile 1 hi, lo
 constexpr int MAX_BSTAGES = 4;
-constexpr int BIAS_REC = 528;              // per N tile: b (2 x 64 floats), c (2 floats), pad
-constexpr int BIAS_SLOTS = 8;              // bias ring depth
+constexpr int BIAS_REC = 528;              // per N tile: b (128 floats), c (one per cluster), pad
 constexpr int MMA_WARPS = 2;               // one MMA issuer per 128-point half
 constexpr int DRAIN_WARPS = 16;            // (lane quarter, cluster of the N tile, half)
 constexpr int WARP_MMA0 = 1, WARP_DRAIN0 = WARP_MMA0 + MMA_WARPS;
@@ -81,53 +80,87 @@ __global__ void k_pack_b(const float* __restrict__ Wt, int K, int Dp, int NT, in
     *reinterpret_cast<uint4*>(base + B_BYTES + off) = *reinterpret_cast<const uint4*>(lo);
 }
 
-// Bias records: per N tile t, b of clusters 2t and 2t+1 (64 floats each, zero past Dp / K) and
-// their constants c (slot 3k of cvec), so the drain reads them from shared memory.
-__global__ void k_pack_bias(const float* __restrict__ bvec, const float* __restrict__ cvec, int K, int Dp, int NT,
+// Bias records: per N tile, b of its clusters (zero past Dp / K) and their constants c (slot 3k of cvec), so the
+// drain reads them from shared memory.
+// W: columns per cluster (64, or 32 in the half-width operands of Dp = 32)
+__global__ void k_pack_bias(const float* __restrict__ bvec, const float* __restrict__ cvec, int K, int Dp, int W, int NT,
                             uint8_t* __restrict__ Bbias)
 {
+    const int CPT = BN / W;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;   // (t, i)
     if (e >= NT * (BIAS_REC / 4)) return;
     const int t = e / (BIAS_REC / 4), i = e % (BIAS_REC / 4);
     float v = 0.f;
-    if (i < 2 * KD) {
-        const int k = CPT * t + i / KD, j = i % KD;
+    if (i < BN) {
+        const int k = CPT * t + i / W, j = i % W;
         if (k < K && j < Dp) v = bvec[(size_t)3 * k * Dp + j];
-    } else if (i < 2 * KD + CPT) {
-        const int k = CPT * t + (i - 2 * KD);
+    } else if (i < BN + CPT) {
+        const int k = CPT * t + (i - BN);
         if (k < K) v = cvec[3 * k];
     }
     reinterpret_cast<float*>(Bbias + (size_t)t * BIAS_REC)[i] = v;
 }
 
+// Operands of the dense label kernel by padded dimension.  DP = 64: a row of 64 BF16 per point / factor column, one
+// image of hi and one of lo; an N tile holds two clusters.  DP = 32: one image whose rows are [32 hi | 32 lo]; an N
+// tile holds four clusters.  A quarter of the products and half the bytes of the zero-padded 64-wide form, whose
+// extra products were all zeros (N = 1e6, K = 20: 414 -> 204 us; what is left is the
+// drain).
+template <int DP>
+struct LabelOps {
+    static constexpr int CPT = BN / DP;                                // clusters per N tile
+    static constexpr uint32_t A = DP == 64 ? A_TILE : A_BYTES;         // bytes per 128 points
+    static constexpr uint32_t B = DP == 64 ? STAGE_BYTES : B_BYTES;    // bytes per N tile
+    static constexpr int KS = DP / 16;                                 // K steps of one product
+    // descriptor distance (16-byte units) from the hi to the lo part
+    static constexpr uint32_t A_LO = DP == 64 ? A_BYTES >> 4 : 64 >> 4, B_LO = DP == 64 ? B_BYTES >> 4 : 64 >> 4;
+    __device__ static uint32_t hi(int row, int k) { return sw128_offset(row, k); }
+    __device__ static uint32_t lo(int row, int k) { return DP == 64 ? A_BYTES + sw128_offset(row, k) : sw128_offset(row, 32 + k); }
+};
+static_assert(A_BYTES == B_BYTES, "one lo distance serves both operands");
+
 // ------------------------------------------------------------------------- A packing
-// Apack[t] = 32 KB: hi (16 KB) then lo (16 KB) of the 128 x 64 K-major swizzled tile holding the
-// points 128t .. 128t+127 (zero rows past N, zero columns past Dp).  The points never change
-// during a run, so the split is done once at upload.
-__global__ void k_pack_a(const float* __restrict__ x, int64_t N, int Dp, int64_t ntiles, uint8_t* __restrict__ Apack)
+// Apack[t]: the rows of the points 128t .. 128t+127 (zero past N) as LabelOps<DP> lays them out, K-major, swizzled.
+// The points never change during a run, so the split is done once at upload.
+template <int DP>
+__global__ void k_pack_a(const float* __restrict__ x, int64_t N, int64_t ntiles, uint8_t* __restrict__ Apack)
 {
+    constexpr int CH = DP / 8;
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;   // (tile, row, chunk)
-    if (e >= ntiles * BM * 8) return;
-    const int64_t t = e / (BM * 8);
-    const int row = (int)((e / 8) % BM), ch = (int)(e % 8);
+    if (e >= ntiles * BM * CH) return;
+    const int64_t t = e / (BM * CH);
+    const int row = (int)((e / CH) % BM), ch = (int)(e % CH);
     const int64_t pt = t * BM + row;
-    float v[8];
-    if (pt < N && ch * 8 < Dp) {
-        const float4* src = reinterpret_cast<const float4*>(x + pt * Dp + ch * 8);
-        const float4 a = src[0], b = src[1];
-        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-    } else {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = 0.f;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+    if (pt < N) {
+        const float4* src = reinterpret_cast<const float4*>(x + pt * DP + ch * 8);
+        a = src[0];
+        b = src[1];
     }
-    __align__(16) __nv_bfloat16 hi[8], lo[8];
+    uint2 h0, l0, h1, l1;
+    bf16_split4(a.x, a.y, a.z, a.w, h0, l0);
+    bf16_split4(b.x, b.y, b.z, b.w, h1, l1);
+    uint8_t* base = Apack + (size_t)t * LabelOps<DP>::A;
+    *reinterpret_cast<uint4*>(base + LabelOps<DP>::hi(row, ch * 8)) = make_uint4(h0.x, h0.y, h1.x, h1.y);
+    *reinterpret_cast<uint4*>(base + LabelOps<DP>::lo(row, ch * 8)) = make_uint4(l0.x, l0.y, l1.x, l1.y);
+}
+
+// B operand at Dp = 32: N tile t = clusters 4t .. 4t + 3, row n = (cluster n / 32, column j = n % 32) -> W(i, j) over i
+__global__ void k_pack_b32(const float* __restrict__ Wt, int K, int NT, uint8_t* __restrict__ Bpack)
+{
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;   // (tile, row, chunk of 8)
+    if (e >= NT * BN * 4) return;
+    const int t = e / (BN * 4), n = (e / 4) % BN, ch = e % 4, k = 4 * t + n / 32;
+    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (k < K)
 #pragma unroll
-    for (int q = 0; q < 8; ++q) bf16_split(v[q], hi[q], lo[q]);
-    uint8_t* base = Apack + (size_t)t * A_TILE;
-    const uint32_t off = sw128_offset(row, ch * 8);
-    *reinterpret_cast<uint4*>(base + off) = *reinterpret_cast<const uint4*>(hi);
-    *reinterpret_cast<uint4*>(base + A_BYTES + off) = *reinterpret_cast<const uint4*>(lo);
+        for (int q = 0; q < 8; ++q) v[q] = Wt[((size_t)3 * k * 32 + n % 32) * 32 + ch * 8 + q];
+    uint2 h0, l0, h1, l1;
+    bf16_split4(v[0], v[1], v[2], v[3], h0, l0);
+    bf16_split4(v[4], v[5], v[6], v[7], h1, l1);
+    uint8_t* base = Bpack + (size_t)t * LabelOps<32>::B;
+    *reinterpret_cast<uint4*>(base + LabelOps<32>::hi(n, ch * 8)) = make_uint4(h0.x, h0.y, h1.x, h1.y);
+    *reinterpret_cast<uint4*>(base + LabelOps<32>::lo(n, ch * 8)) = make_uint4(l0.x, l0.y, l1.x, l1.y);
 }
 
 // ------------------------------------------------------------------------- label kernel
@@ -149,21 +182,20 @@ struct SmemLayout {
     size_t a, b, bias, bar, total;
 };
 
-// mbarrier slots: B ring (full, empty), A slot (afull, aempty), accumulator pairs (tfull,
-// tempty), bias ring (bfull, bempty)
+// mbarrier slots: B ring (full, empty), A slot (afull, aempty), accumulator pairs (tfull, tempty), biases
 constexpr int BAR_FULL = 0, BAR_EMPTY = BAR_FULL + MAX_BSTAGES, BAR_AFULL = BAR_EMPTY + MAX_BSTAGES,
               BAR_AEMPTY = BAR_AFULL + 1, BAR_TFULL = BAR_AEMPTY + 1, BAR_TEMPTY = BAR_TFULL + NPAIR,
-              BAR_BFULL = BAR_TEMPTY + NPAIR, BAR_BEMPTY = BAR_BFULL + BIAS_SLOTS, NBARS = BAR_BEMPTY + BIAS_SLOTS;
-static_assert(NBARS == 30, "barrier slots");
+              BAR_BIAS = BAR_TEMPTY + NPAIR, NBARS = BAR_BIAS + 1;
 
-__host__ __device__ inline SmemLayout smem_layout(int bstages)
+template <int DP>
+__host__ __device__ inline SmemLayout smem_layout(int bstages, int NT)
 {
     SmemLayout L;
     L.bstages = bstages;
-    L.a = 0;                                            // one 64 KB A slot (1024-aligned)
-    L.b = (size_t)A_SLOT;                               // bstages x 32 KB
-    L.bias = L.b + (size_t)bstages * STAGE_BYTES;       // BIAS_SLOTS x BIAS_REC
-    L.bar = L.bias + (size_t)BIAS_SLOTS * BIAS_REC;
+    L.a = 0;                                            // one A slot of two tiles (1024-aligned)
+    L.b = (size_t)HALVES * LabelOps<DP>::A;             // bstages B tiles
+    L.bias = L.b + (size_t)bstages * LabelOps<DP>::B;   // every N tile's record: read by each of its super-tiles
+    L.bar = (L.bias + (size_t)NT * BIAS_REC + 7) / 8 * 8;
     L.total = L.bar + NBARS * 8 + 16 + 1024;            // barriers, tmem slot + flag, alignment slack
     return L;
 }
@@ -173,14 +205,18 @@ __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes)
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
+template <int DP>
 __global__ void __launch_bounds__(THREADS, 1) k_gauss_labels_tc(
     const uint8_t* __restrict__ Apack, int64_t N, int ntiles, const uint8_t* __restrict__ Bpack,
-    const uint8_t* __restrict__ Bbias, int Dp, int K, int bstages, int final_, float* __restrict__ rbuf,
-    float* __restrict__ part, float* __restrict__ r_out, int32_t* __restrict__ err, int stall)
+    const uint8_t* __restrict__ Bbias, int k_first, int K, int bstages, int final_, float* __restrict__ rbuf,
+    float* __restrict__ part, float* __restrict__ r_out, int K_all, int32_t* __restrict__ err, int stall)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    const SmemLayout L = smem_layout(bstages);
+    using O = LabelOps<DP>;
+    constexpr int CPT = O::CPT;
+    const int NT = (K - k_first + CPT - 1) / CPT;   // clusters k_first .. K - 1
+    const SmemLayout L = smem_layout<DP>(bstages, NT);
     uint8_t* sA = smem + L.a;
     uint8_t* sB = smem + L.b;
     uint8_t* sBias = smem + L.bias;
@@ -191,13 +227,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_gauss_labels_tc(
     uint64_t* aempty = bars + BAR_AEMPTY;   // A super-tile consumed
     uint64_t* tfull = bars + BAR_TFULL;     // [NPAIR]     accumulator pair ready
     uint64_t* tempty = bars + BAR_TEMPTY;   // [NPAIR]     accumulator pair drained
-    uint64_t* bfull = bars + BAR_BFULL;     // [BIAS_SLOTS] bias record landed
-    uint64_t* bempty = bars + BAR_BEMPTY;   // [BIAS_SLOTS] bias record read by every drain warp
+    uint64_t* bias_full = bars + BAR_BIAS;  // every bias record landed (once)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NBARS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int NT = (K + CPT - 1) / CPT;
     const int nst = (ntiles + HALVES - 1) / HALVES;
     const volatile int32_t* gerr = err;
 
@@ -213,10 +247,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_gauss_labels_tc(
             mbar_init(&tfull[t], MMA_WARPS);
             mbar_init(&tempty[t], DRAIN_WARPS);
         }
-        for (int s = 0; s < BIAS_SLOTS; ++s) {
-            mbar_init(&bfull[s], 1);
-            mbar_init(&bempty[s], DRAIN_WARPS);
-        }
+        mbar_init(bias_full, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -235,6 +266,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_gauss_labels_tc(
         // ---------------- producer
         if (lane == 0) {
             int gb = 0, la = 0;
+            mbar_arrive_expect_tx(bias_full, (uint32_t)NT * BIAS_REC);
+            bulk_copy_g2s(sBias, Bbias, (uint32_t)NT * BIAS_REC, bias_full);
             for (int st = blockIdx.x; st < nst && !*abort_flag; st += gridDim.x, ++la) {
                 if (!mbar_wait_bounded(aempty, (la & 1) ^ 1, gerr)) {
                     atomicCAS(err, 0, ERR_TIMEOUT_AEMPTY);
@@ -242,30 +275,23 @@ __global__ void __launch_bounds__(THREADS, 1) k_gauss_labels_tc(
                     break;
                 }
                 const int tiles = min(HALVES, ntiles - HALVES * st);
-                const uint32_t abytes = (uint32_t)tiles * A_TILE;
+                const uint32_t abytes = (uint32_t)tiles * O::A;
                 mbar_arrive_expect_tx(afull, abytes);
-                bulk_copy_g2s(sA, Apack + (size_t)HALVES * st * A_TILE, abytes, afull);
+                bulk_copy_g2s(sA, Apack + (size_t)HALVES * st * O::A, abytes, afull);
                 const int nx = st + gridDim.x;   // this CTA's next super-tile: warm L2 for it
                 if (nx < nst)
-                    prefetch_l2(Apack + (size_t)HALVES * nx * A_TILE, (uint32_t)min(HALVES, ntiles - HALVES * nx) * A_TILE);
+                    prefetch_l2(Apack + (size_t)HALVES * nx * O::A, (uint32_t)min(HALVES, ntiles - HALVES * nx) * O::A);
                 bool ok = true;
                 for (int nt = 0; nt < NT; ++nt, ++gb) {
-                    const int s = gb % bstages, sb = gb % BIAS_SLOTS;
-                    if (!mbar_wait_bounded(&empty[s], ((gb / bstages) & 1) ^ 1, gerr)) {
+                    const int s = gb % bstages;
+                    if (!mbar_wait_blocking(&empty[s], ((gb / bstages) & 1) ^ 1, gerr)) {
                         atomicCAS(err, 0, ERR_TIMEOUT_EMPTY);
                         ok = false;   // gb stays the count of B copies issued
                         break;
                     }
-                    if (!mbar_wait_bounded(&bempty[sb], ((gb / BIAS_SLOTS) & 1) ^ 1, gerr)) {
-                        atomicCAS(err, 0, ERR_TIMEOUT_BEMPTY);
-                        ok = false;
-                        break;
-                    }
-                    mbar_arrive_expect_tx(&full[s], STAGE_BYTES);
-                    bulk_copy_g2s(sB + (size_t)s * STAGE_BYTES, Bpack + (size_t)nt * STAGE_BYTES, STAGE_BYTES,
+                    mbar_arrive_expect_tx(&full[s], O::B);
+                    bulk_copy_g2s(sB + (size_t)s * O::B, Bpack + (size_t)nt * O::B, O::B,
                                   &full[s]);
-                    mbar_arrive_expect_tx(&bfull[sb], BIAS_REC);
-                    bulk_copy_g2s(sBias + (size_t)sb * BIAS_REC, Bbias + (size_t)nt * BIAS_REC, BIAS_REC, &bfull[sb]);
                 }
                 if (!ok) {
                     *abort_flag = 1;
@@ -277,8 +303,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_gauss_labels_tc(
             if (la > 0) mbar_wait_bounded(afull, (la - 1) & 1, nullptr);
             for (int q = gb > bstages ? gb - bstages : 0; q < gb; ++q)
                 mbar_wait_bounded(&full[q % bstages], (q / bstages) & 1, nullptr);
-            for (int q = gb > BIAS_SLOTS ? gb - BIAS_SLOTS : 0; q < gb; ++q)
-                mbar_wait_bounded(&bfull[q % BIAS_SLOTS], (q / BIAS_SLOTS) & 1, nullptr);
+            mbar_wait_bounded(bias_full, 0, nullptr);
         }
     } else if (warp < WARP_DRAIN0) {
         // ---------------- MMA issuers: warp WARP_MMA0 + h issues the half-h MMAs of every N tile
@@ -288,10 +313,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_gauss_labels_tc(
         if (lane == 0 && !stall) {
             const int h = warp - WARP_MMA0;
             int g = 0, la = 0, issued = 0;
-            const uint64_t dah = sw128_desc(smem_u32(sA + (size_t)h * A_TILE));
-            const uint64_t dal = sw128_desc(smem_u32(sA + (size_t)h * A_TILE + A_BYTES));
+            const uint64_t dah = sw128_desc(smem_u32(sA + (size_t)h * O::A)), dal = dah + O::A_LO;
             for (int st = blockIdx.x; st < nst && !*abort_flag; st += gridDim.x, ++la) {
-                if (!mbar_wait_bounded(afull, la & 1, gerr)) {
+                if (!mbar_wait_blocking(afull, la & 1, gerr)) {
                     atomicCAS(err, 0, ERR_TIMEOUT_AFULL);
                     *abort_flag = 1;
                     break;
@@ -299,27 +323,26 @@ __global__ void __launch_bounds__(THREADS, 1) k_gauss_labels_tc(
                 bool ok = true;
                 for (int nt = 0; nt < NT; ++nt, ++g) {
                     const int s = g % bstages, t = g % NPAIR;
-                    if (!mbar_wait_bounded(&full[s], (g / bstages) & 1, gerr)) {
+                    if (!mbar_wait_blocking(&full[s], (g / bstages) & 1, gerr)) {
                         atomicCAS(err, 0, ERR_TIMEOUT_FULL);
                         ok = false;
                         break;
                     }
-                    if (!mbar_wait_bounded(&tempty[t], ((g / NPAIR) & 1) ^ 1, gerr)) {
+                    if (!mbar_wait_blocking(&tempty[t], ((g / NPAIR) & 1) ^ 1, gerr)) {
                         atomicCAS(err, 0, ERR_TIMEOUT_TEMPTY);
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t b_hi = smem_u32(sB + (size_t)s * STAGE_BYTES), b_lo = b_hi + B_BYTES;
                     // descriptors: a K step of 16 elements (32 bytes) adds 2 to the start-address field
-                    const uint64_t dbh = sw128_desc(b_hi), dbl = sw128_desc(b_lo);
+                    const uint64_t dbh = sw128_desc(smem_u32(sB + (size_t)s * O::B)), dbl = dbh + O::B_LO;
                     const uint32_t d = tmem_base + (uint32_t)((HALVES * t + h) * BN);
 #pragma unroll
-                    for (int ks = 0; ks < KD / 16; ++ks) umma_bf16(d, dah + 2 * ks, dbh + 2 * ks, ks != 0 ? 1u : 0u);
+                    for (int ks = 0; ks < O::KS; ++ks) umma_bf16(d, dah + 2 * ks, dbh + 2 * ks, ks != 0 ? 1u : 0u);
 #pragma unroll
-                    for (int ks = 0; ks < KD / 16; ++ks) umma_bf16(d, dal + 2 * ks, dbh + 2 * ks, 1u);
+                    for (int ks = 0; ks < O::KS; ++ks) umma_bf16(d, dal + 2 * ks, dbh + 2 * ks, 1u);
 #pragma unroll
-                    for (int ks = 0; ks < KD / 16; ++ks) umma_bf16(d, dah + 2 * ks, dbl + 2 * ks, 1u);
+                    for (int ks = 0; ks < O::KS; ++ks) umma_bf16(d, dah + 2 * ks, dbl + 2 * ks, 1u);
                     umma_commit(&empty[s]);
                     umma_commit(&tfull[t]);
                     issued = g + 1;
@@ -342,6 +365,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_gauss_labels_tc(
         const int p = quarter * 32 + lane;
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
         int g = 0;
+        if (!warp_wait_blocking(bias_full, 0, gerr) && lane == 0) {
+            atomicCAS(err, 0, ERR_TIMEOUT_BFULL);
+            *abort_flag = 1;
+        }
+        __syncwarp();
         for (int st = blockIdx.x; st < nst; st += gridDim.x) {
             if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
             const int64_t pt = ((int64_t)HALVES * st + h) * BM + p;
@@ -349,45 +377,46 @@ __global__ void __launch_bounds__(THREADS, 1) k_gauss_labels_tc(
             float m = -INFINITY, sum = 0.f;   // running max and sum of exp(r - max); final: best, arg
             int arg = -1;
             bool ok = true;
+            if (k_first > 0 && valid) {   // a later pass goes on from the partials of the one before
+                m = part[(size_t)(2 * c) * N + pt];
+                const float q = part[(size_t)(2 * c + 1) * N + pt];
+                if (final_) arg = __float_as_int(q);
+                else sum = q;
+            }
             for (int nt = 0; nt < NT; ++nt, ++g) {
-                const int t = g % NPAIR, sb = g % BIAS_SLOTS;
-                if (!warp_wait_bounded(&tfull[t], (g / NPAIR) & 1, gerr)) {
+                const int t = g % NPAIR;
+                if (!warp_wait_blocking(&tfull[t], (g / NPAIR) & 1, gerr)) {
                     if (lane == 0) atomicCAS(err, 0, ERR_TIMEOUT_TFULL);
                     ok = false;
                     break;
                 }
-                if (!warp_wait_bounded(&bfull[sb], (g / BIAS_SLOTS) & 1, gerr)) {
-                    if (lane == 0) atomicCAS(err, 0, ERR_TIMEOUT_BFULL);
-                    ok = false;
-                    break;
-                }
                 tc_fence_after();
-                const int k = nt * CPT + c;
-                const float* rec = reinterpret_cast<const float*>(sBias + (size_t)sb * BIAS_REC);
-                const float* bk = rec + c * KD;   // b of cluster k; its constant c_k is rec[2 * KD + c]
-                if (k < K) {
-                    // z_j = C[p, j] - b_j over the cluster's 64 columns, in two halves of 32
-                    float q0 = 0.f, q1 = 0.f, q2 = 0.f, q3 = 0.f;
+                const float* rec = reinterpret_cast<const float*>(sBias + (size_t)nt * BIAS_REC);
 #pragma unroll
-                    for (int hh = 0; hh < 2; ++hh) {
-                        if (hh == 1 && Dp <= 32) break;   // columns past Dp are zero
+                for (int cc = 0; cc < CPT / 2; ++cc) {   // this warp's clusters of the tile: one parity, ascending
+                    const int ct = 2 * cc + c, k = k_first + nt * CPT + ct;
+                    if (k >= K) break;
+                    // z_j = C[p, j] - b_j over the cluster's DP columns, 32 at a time; its constant is rec[BN + ct]
+                    const uint64_t minus = pack2(-1.f, -1.f);
+                    uint64_t q01 = 0, q23 = 0;
+#pragma unroll
+                    for (int hh = 0; hh < DP / 32; ++hh) {
                         uint32_t v[32];
-                        tmem_ld32(tmem_base + lane_addr + (uint32_t)((HALVES * t + h) * BN + c * KD + 32 * hh), v);
-                        const float4* b4p = reinterpret_cast<const float4*>(bk + 32 * hh);
+                        tmem_ld32(tmem_base + lane_addr + (uint32_t)((HALVES * t + h) * BN + ct * DP + 32 * hh), v);
+                        const ulonglong2* b4p = reinterpret_cast<const ulonglong2*>(rec + ct * DP + 32 * hh);
 #pragma unroll
                         for (int j4 = 0; j4 < 8; ++j4) {
-                            const float4 b4 = b4p[j4];
-                            const float z0 = __uint_as_float(v[4 * j4 + 0]) - b4.x;
-                            const float z1 = __uint_as_float(v[4 * j4 + 1]) - b4.y;
-                            const float z2 = __uint_as_float(v[4 * j4 + 2]) - b4.z;
-                            const float z3 = __uint_as_float(v[4 * j4 + 3]) - b4.w;
-                            q0 = fmaf(z0, z0, q0);
-                            q1 = fmaf(z1, z1, q1);
-                            q2 = fmaf(z2, z2, q2);
-                            q3 = fmaf(z3, z3, q3);
+                            const ulonglong2 b4 = b4p[j4];
+                            const uint64_t z01 = fma2(b4.x, minus, pack2(__uint_as_float(v[4 * j4]), __uint_as_float(v[4 * j4 + 1])));
+                            const uint64_t z23 = fma2(b4.y, minus, pack2(__uint_as_float(v[4 * j4 + 2]), __uint_as_float(v[4 * j4 + 3])));
+                            q01 = fma2(z01, z01, q01);
+                            q23 = fma2(z23, z23, q23);
                         }
                     }
-                    const float r = rec[2 * KD + c] - 0.5f * ((q0 + q1) + (q2 + q3));
+                    float q0, q1, q2, q3;
+                    unpack2(q01, q0, q1);
+                    unpack2(q23, q2, q3);
+                    const float r = rec[BN + ct] - 0.5f * ((q0 + q1) + (q2 + q3));
                     if (final_) {
                         if (arg < 0 || m < r) { m = r; arg = k; }   // first maximum in cluster order
                     } else {
@@ -399,11 +428,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_gauss_labels_tc(
                         }
                         if (valid) rbuf[(size_t)k * N + pt] = r;
                     }
-                    if (r_out && valid) r_out[pt * K + k] = r;
+                    if (r_out && valid) r_out[pt * K_all + k] = r;
                 }
                 tc_fence_before();
                 warp_arrive(&tempty[t]);
-                if (lane == 0) mbar_arrive(&bempty[sb]);
             }
             if (!ok) {
                 *abort_flag = 1;
@@ -2054,32 +2082,37 @@ __global__ void __launch_bounds__(SS_THREADS, 1) k_sub_stats_tc(
 }  // namespace tc
 
 // B stages: the deepest ring that fits
-static bool tc_config(int& bstages)
+template <int DP>
+static int tc_stages(int K)   // K <= LABEL_PASS: at least two fit
 {
-    for (int bs = tc::MAX_BSTAGES; bs >= 2; --bs)
-        if (tc::smem_layout(bs).total <= tc::kTcSmemCap) {
-            bstages = bs;
-            return true;
-        }
-    return false;
+    int bs = tc::MAX_BSTAGES;
+    while (bs > 2 && tc::smem_layout<DP>(bs, (K * DP + tc::BN - 1) / tc::BN).total > tc::kTcSmemCap) --bs;
+    return bs;
 }
 
 bool tc_supported(const dpmm_ctx* c, int K)
 {
-    int bs = 0;
     return c->prior == DPMM_PRIOR_GAUSSIAN && c->d_Btc != nullptr && c->d_Atc != nullptr && c->d_rbuf != nullptr &&
-           (c->Dp == 32 || c->Dp == 64) && K >= 1 && K <= c->k_max && tc_config(bs);
+           (c->Dp == 32 || c->Dp == 64) && K >= 1 && K <= c->k_max;
 }
 
 // bias records follow the B tiles in the same allocation
 static uint8_t* tc_bias_base(const dpmm_ctx* c)
 {
-    return c->d_Btc + (size_t)((c->k_max + tc::CPT - 1) / tc::CPT) * tc::STAGE_BYTES;
+    return c->Dp == 64 ? c->d_Btc + (size_t)((c->k_max + 1) / 2) * tc::STAGE_BYTES
+                       : c->d_Blab32 + (size_t)((c->k_max + 3) / 4) * tc::LabelOps<32>::B;
 }
 
 size_t tc_param_bytes(int k_max)
 {
     return (size_t)((k_max + tc::CPT - 1) / tc::CPT) * (tc::STAGE_BYTES + tc::BIAS_REC);
+}
+
+size_t tc_param32_bytes(int k_max) { return (size_t)((k_max + 3) / 4) * (tc::LabelOps<32>::B + tc::BIAS_REC); }
+
+size_t tc_point_bytes(int64_t N, int Dp)
+{
+    return (size_t)((N + tc::BM - 1) / tc::BM) * (Dp == 64 ? tc::LabelOps<64>::A : tc::LabelOps<32>::A);
 }
 
 dpmm_status pack_tc_params(dpmm_ctx* c, int K)
@@ -2095,8 +2128,13 @@ dpmm_status pack_tc_params(dpmm_ctx* c, int K)
         tc::k_pack_b<<<(ts + 255) / 256, 256, 0, c->stream>>>(c->d_Wt, K, c->Dp, K, 1, c->d_Bsub);
         DPMM_LAUNCHED();
     }
-    const int nb = NT * (tc::BIAS_REC / 4);
-    tc::k_pack_bias<<<(nb + 255) / 256, 256, 0, c->stream>>>(c->d_b, c->d_c, K, c->Dp, NT, tc_bias_base(c));
+    const int W = c->Dp, NTL = (K * W + tc::BN - 1) / tc::BN;   // N tiles of the label kernel
+    if (c->Dp == 32) {
+        tc::k_pack_b32<<<(NTL * tc::BN * 4 + 255) / 256, 256, 0, c->stream>>>(c->d_Wt, K, NTL, c->d_Blab32);
+        DPMM_LAUNCHED();
+    }
+    const int nb = NTL * (tc::BIAS_REC / 4);
+    tc::k_pack_bias<<<(nb + 255) / 256, 256, 0, c->stream>>>(c->d_b, c->d_c, K, c->Dp, W, NTL, tc_bias_base(c));
     DPMM_LAUNCHED();
     return DPMM_OK;
 }
@@ -2105,32 +2143,43 @@ dpmm_status pack_tc_points(dpmm_ctx* c)
 {
     if (!c->d_Atc) return DPMM_OK;
     const int64_t ntiles = (c->N + tc::BM - 1) / tc::BM;
-    const int64_t total = ntiles * tc::BM * 8;
-    tc::k_pack_a<<<(unsigned)((total + 255) / 256), 256, 0, c->stream>>>(c->d_x, c->N, c->Dp, ntiles, c->d_Atc);
+    const unsigned grid = (unsigned)((ntiles * tc::BM * (c->Dp / 8) + 255) / 256);
+    if (c->Dp == 64) tc::k_pack_a<64><<<grid, 256, 0, c->stream>>>(c->d_x, c->N, ntiles, c->d_Atc);
+    else tc::k_pack_a<32><<<grid, 256, 0, c->stream>>>(c->d_x, c->N, ntiles, c->d_Atc);
     DPMM_LAUNCHED();
+    return DPMM_OK;
+}
+
+template <int DP>
+static dpmm_status launch_labels_tc_t(dpmm_ctx* c, int K, int final_, float* d_rout, int32_t* err)
+{
+    using O = tc::LabelOps<DP>;
+    auto kern = tc::k_gauss_labels_tc<DP>;
+    const int64_t ntiles = (c->N + tc::BM - 1) / tc::BM;
+    const int64_t nst = (ntiles + tc::HALVES - 1) / tc::HALVES;
+    const unsigned grid = (unsigned)std::min<int64_t>(nst, c->num_sms);
+    const uint8_t* B = DP == 64 ? c->d_Btc : c->d_Blab32;
+    KernelTimer kt(c, PH_LABEL_KERNEL);
+    for (int k0 = 0; k0 < K; k0 += tc::LABEL_PASS) {
+        const int k1 = std::min(K, k0 + tc::LABEL_PASS), bstages = tc_stages<DP>(k1 - k0);
+        const tc::SmemLayout L = tc::smem_layout<DP>(bstages, (k1 - k0 + O::CPT - 1) / O::CPT);
+        DPMM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total));
+        kern<<<grid, tc::THREADS, L.total, c->stream>>>(c->d_Atc, c->N, (int)ntiles, B + (size_t)(k0 / O::CPT) * O::B,
+                                                        tc_bias_base(c) + (size_t)(k0 / O::CPT) * tc::BIAS_REC, k0, k1,
+                                                        bstages, final_, c->d_rbuf, c->d_rpart, d_rout, K, err,
+                                                        c->stall_tc_mma);
+        DPMM_LAUNCHED();
+    }
     return DPMM_OK;
 }
 
 dpmm_status launch_cluster_labels_tc(dpmm_ctx* c, int K, int final_, const float* d_u, float* d_rout)
 {
-    int bstages = 0;
-    if (!tc_supported(c, K) || !tc_config(bstages))
-        return fail(DPMM_ERR_INVALID_ARG, "tensor-core label kernel: unsupported shape");
-    const tc::SmemLayout L = tc::smem_layout(bstages);
-    DPMM_CUDA_TRY(cudaFuncSetAttribute(tc::k_gauss_labels_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total));
+    if (!tc_supported(c, K)) return fail(DPMM_ERR_INVALID_ARG, "tensor-core label kernel: unsupported shape");
     int32_t* err = c->d_aux + 4;
     DPMM_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int32_t), c->stream));
-    const int64_t ntiles = (c->N + tc::BM - 1) / tc::BM;
-    const int64_t nst = (ntiles + tc::HALVES - 1) / tc::HALVES;
-    const unsigned grid = (unsigned)std::min<int64_t>(nst, c->num_sms);
-    {
-        KernelTimer kt(c, PH_LABEL_KERNEL);
-        tc::k_gauss_labels_tc<<<grid, tc::THREADS, L.total, c->stream>>>(c->d_Atc, c->N, (int)ntiles, c->d_Btc,
-                                                                         tc_bias_base(c), c->Dp, K, bstages, final_,
-                                                                         c->d_rbuf, c->d_rpart, d_rout, err,
-                                                                         c->stall_tc_mma);
-        DPMM_LAUNCHED();
-    }
+    if (c->Dp == 64) DPMM_TRY(launch_labels_tc_t<64>(c, K, final_, d_rout, err));
+    else DPMM_TRY(launch_labels_tc_t<32>(c, K, final_, d_rout, err));
     RngArgs r = rng_args(c, d_u);
     DPMM_TRY(tc::launch_draw_labels(c, K, final_, r));
     int32_t h_err = 0;

@@ -140,6 +140,16 @@ __device__ __forceinline__ bool warp_wait_bounded(uint64_t* bar, uint32_t parity
     return ok != 0;
 }
 
+// The same on the blocking probe.
+__device__ __forceinline__ bool warp_wait_blocking(uint64_t* bar, uint32_t parity, const volatile int32_t* gerr)
+{
+    int ok = 1;
+    if ((threadIdx.x & 31) == 0) ok = mbar_wait_blocking(bar, parity, gerr) ? 1 : 0;
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+    __syncwarp();
+    return ok != 0;
+}
+
 // One arrival per warp: every lane's prior work is ordered before lane 0's release by __syncwarp.
 __device__ __forceinline__ void warp_arrive(uint64_t* bar)
 {
