@@ -425,13 +425,4 @@ __device__ __forceinline__ int alias_draw_y(const YF& y, const SF& flags, int K,
     return alias_merge(y, K, ns, ReadFlags<YF>{y, K}, u1, u2);
 }
 
-// y stored in memory: ys[(k - 1) * stride] for category k.
-__device__ __forceinline__ int alias_draw_stream(const float* __restrict__ ys, int64_t stride, int K, float u1,
-                                                 float u2)
-{
-    auto y = [=](int i) -> float { return ys[(size_t)i * stride]; };
-    auto flags = [=](int i) -> uint32_t { return ys[(size_t)i * stride] < 1.f ? 3u : 0u; };
-    return alias_draw_y(y, flags, K, u1, u2);
-}
-
 }  // namespace dpmm

@@ -15,8 +15,13 @@
 #include <vector>
 
 #include "dpmm_device.cuh"
+#include "dpmm_tc.cuh"
 
 namespace dpmm {
+
+using tc::fma2;
+using tc::pack2;
+using tc::unpack2;
 
 RngArgs rng_args(dpmm_ctx* c, const float* d_ucaller)
 {
@@ -126,99 +131,135 @@ __device__ __forceinline__ int draw_from_r(float* sr, int p, int K, int final_, 
     }
     const float inv = 1.0f / sum;
     const float fk = (float)K;
-    for (int k = 0; k < K; ++k) sr[k * P + p] = (sr[k * P + p] * inv) * fk;   // y_k = p_k * K
+    const float* e = sr + p;
+    auto y = [=](int k) -> float { return (e[k * P] * inv) * fk; };   // y_k = p_k * K, made where it is read
+    auto flags = [=](int k) -> uint32_t { return y(k) < 1.f ? 3u : 0u; };
     float u1, u2;
     draw_uniform2(rng, pt, u1, u2);
-    return alias_draw_stream(sr + p, P, K, u1, u2);
+    return alias_draw_y(y, flags, K, u1, u2);
 }
 
 // Gaussian label phase, FP32 SIMT: one thread per point, x in registers, each cluster's
 // precision factor (transposed) broadcast from shared memory.
 //   z_j = sum_i W(i,j) x_i - b_j,   r_k = c_k - 0.5 * sum_j z_j^2
-// r = c - 0.5 |W^T x - b|^2 for one point (x in registers) and one cluster whose transposed factor
-// (Wt[j][i] = W(i, j)) and b are staged in shared memory
+// r = c - 0.5 |W^T x - b|^2 for one point (x in registers, two features to a 64-bit pair) and one cluster whose
+// transposed factor (Wt[j][i] = W(i, j)) and b are staged in shared memory.  z_j is the sum of an even-feature and an
+// odd-feature chain, one packed multiply-add for both.
 template <int DP>
-__device__ __forceinline__ float gauss_r_point(const float* __restrict__ sW, const float* __restrict__ sbv,
-                                               const float (&xr)[DP], float c)
+__device__ __forceinline__ float gauss_r_pairs(const float* __restrict__ sW, const float* __restrict__ sbv,
+                                               const uint64_t (&x2)[DP / 2], float c)
 {
     float q = 0.f;
 #pragma unroll 2
     for (int j = 0; j < DP; j += 2) {
-        const float4* w0 = reinterpret_cast<const float4*>(sW + j * DP);
-        const float4* w1 = reinterpret_cast<const float4*>(sW + (j + 1) * DP);
-        float z0 = -sbv[j], z1 = -sbv[j + 1];
-        float z0b = 0.f, z1b = 0.f;
+        const ulonglong2* w0 = reinterpret_cast<const ulonglong2*>(sW + j * DP);
+        const ulonglong2* w1 = reinterpret_cast<const ulonglong2*>(sW + (j + 1) * DP);
+        uint64_t z0 = pack2(-sbv[j], 0.f), z1 = pack2(-sbv[j + 1], 0.f);
 #pragma unroll
         for (int i4 = 0; i4 < DP / 4; ++i4) {
-            float4 a = w0[i4], b = w1[i4];
-            z0 = fmaf(a.x, xr[4 * i4 + 0], z0);
-            z1 = fmaf(b.x, xr[4 * i4 + 0], z1);
-            z0b = fmaf(a.y, xr[4 * i4 + 1], z0b);
-            z1b = fmaf(b.y, xr[4 * i4 + 1], z1b);
-            z0 = fmaf(a.z, xr[4 * i4 + 2], z0);
-            z1 = fmaf(b.z, xr[4 * i4 + 2], z1);
-            z0b = fmaf(a.w, xr[4 * i4 + 3], z0b);
-            z1b = fmaf(b.w, xr[4 * i4 + 3], z1b);
+            const ulonglong2 a = w0[i4], b = w1[i4];
+            z0 = fma2(a.x, x2[2 * i4], z0);
+            z1 = fma2(b.x, x2[2 * i4], z1);
+            z0 = fma2(a.y, x2[2 * i4 + 1], z0);
+            z1 = fma2(b.y, x2[2 * i4 + 1], z1);
         }
-        z0 += z0b;
-        z1 += z1b;
-        q = fmaf(z0, z0, q);
-        q = fmaf(z1, z1, q);
+        float e, o;
+        unpack2(z0, e, o);
+        e += o;
+        q = fmaf(e, e, q);
+        unpack2(z1, e, o);
+        e += o;
+        q = fmaf(e, e, q);
     }
     return c - 0.5f * q;
 }
 
-// one block of P points starting at pt0 (the body of k_gauss_labels_simt and of its batched form)
+template <int DP>
+__device__ __forceinline__ float gauss_r_point(const float* __restrict__ sW, const float* __restrict__ sbv,
+                                               const float (&xr)[DP], float c)
+{
+    uint64_t x2[DP / 2];
+#pragma unroll
+    for (int i = 0; i < DP / 2; ++i) x2[i] = pack2(xr[2 * i], xr[2 * i + 1]);
+    return gauss_r_pairs<DP>(sW, sbv, x2, c);
+}
+
+constexpr size_t kLabelSmemCap = 220 * 1024;
+
+// Shape of the label kernel for blocks of P points: a thread per point and KB clusters staged between two barriers
+// (16 KB of factors, at least one cluster).  At N = 1e6, D = 7, K = 30 this takes 215 us; two points per thread took
+// 190, but in batches of small data sets 117 against 48, and reading the factors through the L1 cache 284.
+template <int DP, int P>
+struct LabelTile {
+    static constexpr int KB = DP * DP * 4 >= 16384 ? 1 : 16384 / (DP * DP * 4);
+    static constexpr int F4 = DP * DP / 4;
+    // shared memory in bytes: kb factors and biases, then r [K][P]; kb: KB, or what the cap leaves beside a large K
+    static size_t bytes(int K, int kb) { return sizeof(float) * ((size_t)kb * (DP * DP + DP) + (size_t)K * P); }
+    static int staged(int K)
+    {
+        int kb = KB < K ? KB : K;
+        while (kb > 1 && bytes(K, kb) > kLabelSmemCap) --kb;
+        return kb;
+    }
+};
+
+// one block of P points starting at pt0 (the body of k_gauss_labels_simt and of its batched form).  Bound: reads of
+// the factors from shared memory (16 bytes for two packed multiply-adds and point) and, where the clusters overlap,
+// the draws.  Barriers come once per KB clusters and the points go straight to registers, so that several blocks
+// fit an SM: N = 1e5, D = 100, K = 12 2200 -> 1320 us; N = 1e6, D = 7, K = 30 236 -> 215 us.
 template <int DP, int P>
 __device__ __forceinline__ void gauss_labels_tile(const float* __restrict__ x, int64_t N,
                                                   const float* __restrict__ Wt, const float* __restrict__ bvec,
                                                   const float* __restrict__ cvec, int K, int final_,
                                                   const RngArgs& rng, int32_t* __restrict__ labels,
-                                                  float* __restrict__ r_out, int64_t pt0, unsigned char* smem)
+                                                  float* __restrict__ r_out, int64_t pt0, int kb,
+                                                  unsigned char* smem)
 {
-    float* sW = reinterpret_cast<float*>(smem);          // DP*DP
-    float* sbv = sW + DP * DP;                            // DP
-    float* sx = sbv + DP;                                 // P*(DP+1)
-    float* sr = sx + P * (DP + 1);                        // K*P
+    using L = LabelTile<DP, P>;
+    float* sW = reinterpret_cast<float*>(smem);           // kb * DP*DP
+    float* sbv = sW + (size_t)kb * DP * DP;               // kb * DP
+    float* sr = sbv + (size_t)kb * DP;                    // K*P
 
-    const int p = threadIdx.x;
-    const int64_t pt = pt0 + p;
+    const int t = threadIdx.x;
+    const int64_t pt = pt0 + t;
     const bool valid = pt < N;
-
-    // stage the tile's points (contiguous rows) with coalesced loads
-    const int64_t rows = min((int64_t)P, N - pt0);
-    for (int e = p; e < P * DP; e += P) {
-        int pp = e / DP, i = e % DP;
-        sx[pp * (DP + 1) + i] = pp < rows ? x[(pt0 + pp) * DP + i] : 0.f;
-    }
-    __syncthreads();
-    float xr[DP];
+    uint64_t x2[DP / 2];
+    {
+        const ulonglong2* src = reinterpret_cast<const ulonglong2*>(x + min(pt, N - 1) * DP);
 #pragma unroll
-    for (int i = 0; i < DP; ++i) xr[i] = sx[p * (DP + 1) + i];
-
-    for (int k = 0; k < K; ++k) {
-        __syncthreads();
-        const float4* src = reinterpret_cast<const float4*>(Wt + (size_t)3 * k * DP * DP);
-        float4* dst = reinterpret_cast<float4*>(sW);
-        for (int e = p; e < DP * DP / 4; e += P) dst[e] = src[e];
-        for (int e = p; e < DP; e += P) sbv[e] = bvec[(size_t)3 * k * DP + e];
-        __syncthreads();
-        const float r = gauss_r_point<DP>(sW, sbv, xr, cvec[3 * k]);
-        sr[k * P + p] = r;
-        if (r_out && valid) r_out[pt * K + k] = r;
+        for (int i4 = 0; i4 < DP / 4; ++i4) {
+            const ulonglong2 v = __ldg(src + i4);
+            x2[2 * i4] = v.x;
+            x2[2 * i4 + 1] = v.y;
+        }
     }
-    if (!valid) return;
-    labels[pt] = draw_from_r<P>(sr, p, K, final_, rng, pt);
+    for (int k0 = 0; k0 < K; k0 += kb) {
+        const int nk = min(kb, K - k0);
+        __syncthreads();
+        for (int e = t; e < nk * L::F4; e += P) {
+            const int kk = e / L::F4;
+            reinterpret_cast<float4*>(sW)[e] = reinterpret_cast<const float4*>(Wt + (size_t)3 * (k0 + kk) * DP * DP)[e % L::F4];
+        }
+        for (int e = t; e < nk * DP; e += P) sbv[e] = bvec[(size_t)3 * (k0 + e / DP) * DP + e % DP];
+        __syncthreads();
+        for (int kk = 0; kk < nk; ++kk) {
+            const int k = k0 + kk;
+            const float r = gauss_r_pairs<DP>(sW + (size_t)kk * DP * DP, sbv + kk * DP, x2, cvec[3 * k]);
+            sr[k * P + t] = r;
+            if (r_out && valid) r_out[pt * K + k] = r;
+        }
+    }
+    if (valid) labels[pt] = draw_from_r<P>(sr, t, K, final_, rng, pt);
 }
 
 template <int DP, int P>
 __global__ void __launch_bounds__(P) k_gauss_labels_simt(
     const float* __restrict__ x, int64_t N, const float* __restrict__ Wt, const float* __restrict__ bvec,
     const float* __restrict__ cvec, int K, int final_, RngArgs rng, int32_t* __restrict__ labels,
-    float* __restrict__ r_out)
+    float* __restrict__ r_out, int kb)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    gauss_labels_tile<DP, P>(x, N, Wt, bvec, cvec, K, final_, rng, labels, r_out, (int64_t)blockIdx.x * P, smem);
+    gauss_labels_tile<DP, P>(x, N, Wt, bvec, cvec, K, final_, rng, labels, r_out, (int64_t)blockIdx.x * P, kb, smem);
 }
 
 // Batched form: one launch for many data sets of the same padded dimension.  Block b works on
@@ -226,15 +267,16 @@ __global__ void __launch_bounds__(P) k_gauss_labels_simt(
 // stream come from its descriptor.  Shared memory is sized for the largest K of the batch.
 template <int DP, int P>
 __global__ void __launch_bounds__(P) k_gauss_labels_batched(const LabelJob* __restrict__ jobs,
-                                                            const int2* __restrict__ items)
+                                                            const int2* __restrict__ items, int kb)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int2 it = items[blockIdx.x];
     const LabelJob& j = jobs[it.x];
     gauss_labels_tile<DP, P>(j.x, j.N, j.Wt, j.b, j.c, j.K, j.final_, j.rng, j.labels, nullptr, (int64_t)it.y * P,
-                             smem);
+                             kb, smem);
 }
 
+// the batch's capacity rule (more than any block here needs)
 size_t gauss_label_smem_bytes(int DP, int P, int K)
 {
     return sizeof(float) * (DP * DP + DP + P * (DP + 1) + (size_t)K * P);
@@ -244,11 +286,12 @@ template <int DP, int P>
 static dpmm_status launch_labels_batched_t(const LabelJob* d_jobs, const int2* d_items, int nitems, int kmax,
                                            cudaStream_t st)
 {
-    const size_t sm = gauss_label_smem_bytes(DP, P, kmax);
-    if (sm > 220 * 1024) return fail(DPMM_ERR_INVALID_ARG, "too many clusters for the batched label kernel");
+    if (gauss_label_smem_bytes(DP, P, kmax) > kLabelSmemCap) return fail(DPMM_ERR_INVALID_ARG, "too many clusters for the batched label kernel");
+    const int kb = LabelTile<DP, P>::staged(kmax);
+    const size_t sm = LabelTile<DP, P>::bytes(kmax, kb);
     auto kern = k_gauss_labels_batched<DP, P>;
     DPMM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    kern<<<nitems, P, sm, st>>>(d_jobs, d_items);
+    kern<<<nitems, P, sm, st>>>(d_jobs, d_items, kb);
     DPMM_LAUNCHED();
     return DPMM_OK;
 }
@@ -343,19 +386,15 @@ __global__ void __launch_bounds__(256) k_mult_labels_simt(
     labels[pt] = draw_from_r<P>(sr, tid, K, final_, rng, pt);
 }
 
-static size_t gauss_label_smem(int DP, int P, int K)
-{
-    return sizeof(float) * (DP * DP + DP + P * (DP + 1) + (size_t)K * P);
-}
-
 template <int DP, int P>
 static dpmm_status launch_gauss_labels_t(dpmm_ctx* c, int K, int final_, RngArgs r, float* d_rout)
 {
-    const size_t sm = gauss_label_smem(DP, P, K);
+    const int kb = LabelTile<DP, P>::staged(K);
+    const size_t sm = LabelTile<DP, P>::bytes(K, kb);
     auto kern = k_gauss_labels_simt<DP, P>;
     DPMM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     kern<<<blocks_for(c->N, P), P, sm, c->stream>>>(c->d_x, c->N, c->d_Wt, c->d_b, c->d_c, K, final_, r,
-                                                     c->d_labels, d_rout);
+                                                     c->d_labels, d_rout, kb);
     DPMM_LAUNCHED();
     return DPMM_OK;
 }
@@ -363,10 +402,9 @@ static dpmm_status launch_gauss_labels_t(dpmm_ctx* c, int K, int final_, RngArgs
 template <int DP>
 static dpmm_status launch_gauss_labels_dp(dpmm_ctx* c, int K, int final_, RngArgs r, float* d_rout)
 {
-    const size_t cap = 220 * 1024;
-    if (gauss_label_smem(DP, 128, K) <= cap) return launch_gauss_labels_t<DP, 128>(c, K, final_, r, d_rout);
-    if (gauss_label_smem(DP, 64, K) <= cap) return launch_gauss_labels_t<DP, 64>(c, K, final_, r, d_rout);
-    if (gauss_label_smem(DP, 32, K) <= cap) return launch_gauss_labels_t<DP, 32>(c, K, final_, r, d_rout);
+    if (gauss_label_smem_bytes(DP, 128, K) <= kLabelSmemCap) return launch_gauss_labels_t<DP, 128>(c, K, final_, r, d_rout);
+    if (gauss_label_smem_bytes(DP, 64, K) <= kLabelSmemCap) return launch_gauss_labels_t<DP, 64>(c, K, final_, r, d_rout);
+    if (gauss_label_smem_bytes(DP, 32, K) <= kLabelSmemCap) return launch_gauss_labels_t<DP, 32>(c, K, final_, r, d_rout);
     return fail(DPMM_ERR_INVALID_ARG, "too many clusters for the label kernel's shared-memory table");
 }
 
