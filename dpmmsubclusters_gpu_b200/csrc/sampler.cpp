@@ -1487,6 +1487,7 @@ struct dpmm_batch {
         cudaEvent_t done = nullptr;
         cudaGraphExec_t graph = nullptr;
         float tune_ms[3] = {0, 0, 0};
+        int tuned_K = 0;               // largest K of the jobs it was timed on
     };
     std::vector<std::unique_ptr<dpmm::host::SamplerHandle>> s;
     std::vector<Group> groups;
@@ -1542,9 +1543,12 @@ static dpmm_status batch_labels(dpmm_batch& b, dpmm_batch::Group& g, const std::
         DPMM_TRY(make_label_job(sm.context(), sm.num_clusters(), st[mem[j]].final_ ? 1 : 0, &g.h_jobs[j]));
     }
     const size_t jb = sizeof(LabelJob) * mem.size();
-    if (g.P == 0) {
-        // first iteration: time every block size on the live jobs (each run draws the same labels:
-        // a point's log-likelihoods and uniforms do not depend on the block size), keep the fastest
+    int kmax = 1;
+    for (size_t j = 0; j < mem.size(); ++j) kmax = std::max(kmax, g.h_jobs[j].K);
+    if (g.P == 0 || kmax >= 2 * g.tuned_K) {
+        // first iteration, and whenever the largest job has doubled its clusters since (what one cluster
+        // favours, the staging of many punishes): time every block size on the live jobs (each run draws the
+        // same labels: a point's log-likelihoods and uniforms do not depend on the block size), keep the fastest
         cudaEvent_t e0, e1;
         DPMM_CUDA_TRY(cudaEventCreate(&e0));
         DPMM_CUDA_TRY(cudaEventCreate(&e1));
@@ -1563,6 +1567,11 @@ static dpmm_status batch_labels(dpmm_batch& b, dpmm_batch::Group& g, const std::
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         g.P = kBatchP[best];
+        g.tuned_K = kmax;
+        if (g.graph) {
+            cudaGraphExecDestroy(g.graph);
+            g.graph = nullptr;
+        }
         DPMM_TRY(batch_items(b, g, mem, g.P));
         return DPMM_OK;
     }
