@@ -1125,24 +1125,22 @@ dpmm_status build_permutation(dpmm_ctx* c, int K)
 // per sub-cluster: count, sum(x - s) and the upper triangle of sum (x - s)(x - s)^T, shift
 // s = the cluster's mean parameter.  FP32 products, FP32 runs of at most 33 points, FP64 totals.
 //
-// DP <= 64 ("blocked" form, 128 points per tile):
+// DP <= 64, 128 points per tile (the two kernels below take DP = 128):
 //   draw  - two threads per point, one per side: warps 0-3 evaluate the l factor, warps 4-7 the r
 //           factor, x in registers, factor rows broadcast from shared memory as float4;
 //   stats - each thread of a warp-aligned group owns one 4 x 4 block of the upper triangle and
 //           does 16 FMAs per point from two float4 loads; G groups take every G-th point of the
 //           tile; FP64 totals per thread live in shared memory and are summed over the groups at
 //           the end.
-// DP = 128: one thread per point for the draw, one matrix entry per thread through a pair table.
 
 template <int DP>
 struct SubStatsShape {
-    static constexpr bool BLOCKED = DP <= 64;
     static constexpr int TP = 128;                                   // points per tile
     static constexpr int SX = DP + 4;                                // shared row stride (16-byte rows)
     static constexpr int NB = DP / 4;
     static constexpr int NBLK = NB * (NB + 1) / 2;                   // 4 x 4 blocks of the triangle
     static constexpr int GS = (NBLK + 31) / 32 * 32;                 // threads per group (whole warps)
-    static constexpr int G = BLOCKED ? 256 / GS : 1;                 // groups
+    static constexpr int G = 256 / GS;                 // groups
     static constexpr int NTOT = G * NBLK;                            // owners of FP64 totals
     // shared layout in bytes
     static constexpr size_t off_wl = 0;
@@ -1153,16 +1151,14 @@ struct SubStatsShape {
     static constexpr size_t off_x = (off_s + sizeof(float) * DP + 15) / 16 * 16;
     static constexpr size_t off_q = off_x + sizeof(float) * TP * SX;
     static constexpr size_t off_sub = off_q + sizeof(float) * 2 * TP;
-    static constexpr size_t off_tail = (off_sub + sizeof(int32_t) * TP + 15) / 16 * 16;
-    // blocked: FP64 block totals [32][NTOT] then sums [G][2][DP]; DP = 128: pair table
-    static constexpr size_t off_tot = off_tail;
-    static constexpr size_t off_sum = off_tot + (BLOCKED ? sizeof(double) * 32 * NTOT : 0);
-    static constexpr size_t bytes = BLOCKED ? off_sum + sizeof(double) * G * 2 * DP
-                                            : off_tail + sizeof(uint16_t) * tri(DP);
+    // FP64 block totals [32][NTOT], then sums [G][2][DP]
+    static constexpr size_t off_tot = (off_sub + sizeof(int32_t) * TP + 15) / 16 * 16;
+    static constexpr size_t off_sum = off_tot + sizeof(double) * 32 * NTOT;
+    static constexpr size_t bytes = off_sum + sizeof(double) * G * 2 * DP;
 };
 
 template <int DP>
-__global__ void __launch_bounds__(256, (DP >= 128 ? 1 : 2)) k_gauss_sub_stats(
+__global__ void __launch_bounds__(256, 2) k_gauss_sub_stats(
     const float* __restrict__ x, const int32_t* __restrict__ perm, const int32_t* __restrict__ chunk,
     const int32_t* __restrict__ nchunks, const float* __restrict__ Wt, const float* __restrict__ bvec,
     const float* __restrict__ cvec, const float* __restrict__ lrw, const float* __restrict__ muv, int draw,
@@ -1173,7 +1169,6 @@ __global__ void __launch_bounds__(256, (DP >= 128 ? 1 : 2)) k_gauss_sub_stats(
     constexpr int T = tri(DP);
     constexpr int SL = 1 + DP + T;            // partial record length per sub-cluster
     constexpr int TP = S::TP, SX = S::SX;
-    constexpr int E = S::BLOCKED ? 1 : (T + 255) / 256;
     extern __shared__ __align__(16) unsigned char smem[];
     float* sWl = reinterpret_cast<float*>(smem + S::off_wl);
     float* sWr = reinterpret_cast<float*>(smem + S::off_wr);
@@ -1185,7 +1180,6 @@ __global__ void __launch_bounds__(256, (DP >= 128 ? 1 : 2)) k_gauss_sub_stats(
     int32_t* ssub = reinterpret_cast<int32_t*>(smem + S::off_sub);
     double* stot = reinterpret_cast<double*>(smem + S::off_tot);
     double* ssum = reinterpret_cast<double*>(smem + S::off_sum);
-    uint16_t* spair = reinterpret_cast<uint16_t*>(smem + S::off_tail);
 
     const int ch = blockIdx.x;
     if (ch >= *nchunks) return;
@@ -1218,19 +1212,12 @@ __global__ void __launch_bounds__(256, (DP >= 128 ? 1 : 2)) k_gauss_sub_stats(
             (tid < DP ? sbl : sbr)[j] -= acc;
         }
     }
-    if constexpr (!S::BLOCKED) {
-        for (int e = tid; e < T; e += 256) {
-            int i = 0, rem = e;
-            while (rem >= DP - i) { rem -= DP - i; ++i; }
-            spair[e] = (uint16_t)((i << 8) | (i + rem));
-        }
-    }
     const float cl = draw ? cvec[3 * k + 1] : 0.f, cr = draw ? cvec[3 * k + 2] : 0.f;
     const float wl = draw ? lrw[2 * k] : 0.f, wr = draw ? lrw[2 * k + 1] : 0.f;
 
-    // blocked form: this thread's group, 4 x 4 block (bi <= bj) and FP64 total column
+    // this thread's group, 4 x 4 block (bi <= bj) and FP64 total column
     const int grp = tid / S::GS, tb = tid % S::GS;
-    const bool has_blk = S::BLOCKED && grp < S::G && tb < S::NBLK;
+    const bool has_blk = grp < S::G && tb < S::NBLK;
     int bi = 0, bj = 0;
     if (has_blk) {
         int rem = tb;
@@ -1239,55 +1226,38 @@ __global__ void __launch_bounds__(256, (DP >= 128 ? 1 : 2)) k_gauss_sub_stats(
     }
     const bool diag = has_blk && bi == bj;
     const int tcol = grp * S::NBLK + tb;
-    if constexpr (S::BLOCKED) {
-        if (has_blk)
-            for (int m = 0; m < 32; ++m) stot[m * S::NTOT + tcol] = 0.0;
-        for (int e = tid; e < S::G * 2 * DP; e += 256) ssum[e] = 0.0;
-    }
+    if (has_blk)
+        for (int m = 0; m < 32; ++m) stot[m * S::NTOT + tcol] = 0.0;
+    for (int e = tid; e < S::G * 2 * DP; e += 256) ssum[e] = 0.0;
     float bf[2][16];
     float sf[2][4];
-    float accf[2][E];
-    double accd[2][E];
 #pragma unroll
     for (int s2 = 0; s2 < 2; ++s2) {
 #pragma unroll
         for (int m = 0; m < 16; ++m) bf[s2][m] = 0.f;
 #pragma unroll
         for (int m = 0; m < 4; ++m) sf[s2][m] = 0.f;
-#pragma unroll
-        for (int m = 0; m < E; ++m) { accf[s2][m] = 0.f; accd[s2][m] = 0.0; }
     }
-    float sumf = 0.f;     // DP = 128: threads [0, DP) -> l sums, [DP, 2DP) -> r sums
-    double sumd = 0.0;
     int cnt_l = 0, cnt_r = 0;
 
     auto flush = [&]() {
-        if constexpr (S::BLOCKED) {
-            if (has_blk) {
-#pragma unroll
-                for (int s2 = 0; s2 < 2; ++s2)
-#pragma unroll
-                    for (int m = 0; m < 16; ++m) {
-                        stot[(16 * s2 + m) * S::NTOT + tcol] += (double)bf[s2][m];
-                        bf[s2][m] = 0.f;
-                    }
-                if (diag) {
-#pragma unroll
-                    for (int s2 = 0; s2 < 2; ++s2)
-#pragma unroll
-                        for (int a = 0; a < 4; ++a) {
-                            ssum[(grp * 2 + s2) * DP + 4 * bi + a] += (double)sf[s2][a];
-                            sf[s2][a] = 0.f;
-                        }
-                }
-            }
-        } else {
+        if (has_blk) {
 #pragma unroll
             for (int s2 = 0; s2 < 2; ++s2)
 #pragma unroll
-                for (int m = 0; m < E; ++m) { accd[s2][m] += (double)accf[s2][m]; accf[s2][m] = 0.f; }
-            sumd += (double)sumf;
-            sumf = 0.f;
+                for (int m = 0; m < 16; ++m) {
+                    stot[(16 * s2 + m) * S::NTOT + tcol] += (double)bf[s2][m];
+                    bf[s2][m] = 0.f;
+                }
+            if (diag) {
+#pragma unroll
+                for (int s2 = 0; s2 < 2; ++s2)
+#pragma unroll
+                    for (int a = 0; a < 4; ++a) {
+                        ssum[(grp * 2 + s2) * DP + 4 * bi + a] += (double)sf[s2][a];
+                        sf[s2][a] = 0.f;
+                    }
+            }
         }
     };
 
@@ -1307,11 +1277,9 @@ __global__ void __launch_bounds__(256, (DP >= 128 ? 1 : 2)) k_gauss_sub_stats(
                 pf[u] = __ldg(reinterpret_cast<const float4*>(x + (size_t)__ldg(perm + start + t0 + pp) * DP) + i4);
         }
     };
-    constexpr bool PREFETCH = DP <= 64;             // DP = 128: too many registers, load at the tile start
-    if (PREFETCH) load_tile(0);
+    load_tile(0);
     for (int t0 = 0; t0 < len; t0 += TP) {
         const int nt = min(TP, len - t0);
-        if (!PREFETCH) load_tile(t0);
         __syncthreads();
 #pragma unroll
         for (int u = 0; u < NPF; ++u) {
@@ -1326,63 +1294,41 @@ __global__ void __launch_bounds__(256, (DP >= 128 ? 1 : 2)) k_gauss_sub_stats(
         }
         __syncthreads();
         if (draw) {
-            if constexpr (S::BLOCKED) {
-                // quadratic form of one side for one point
-                const int side = tid >> 7, pp = tid & 127;
-                const float* W = side ? sWr : sWl;
-                const float* bb = side ? sbr : sbl;
-                float xr[DP];
+            // quadratic form of one side for one point
+            const int side = tid >> 7, pp = tid & 127;
+            const float* W = side ? sWr : sWl;
+            const float* bb = side ? sbr : sbl;
+            float xr[DP];
+#pragma unroll
+            for (int i4 = 0; i4 < DP / 4; ++i4) {
+                const float4 v = *reinterpret_cast<const float4*>(sx + pp * SX + 4 * i4);
+                xr[4 * i4] = v.x; xr[4 * i4 + 1] = v.y; xr[4 * i4 + 2] = v.z; xr[4 * i4 + 3] = v.w;
+            }
+            float q0 = 0.f, q1 = 0.f;
+#pragma unroll 2
+            for (int j = 0; j < DP; j += 2) {
+                const float4* w0 = reinterpret_cast<const float4*>(W + j * DP);
+                const float4* w1 = reinterpret_cast<const float4*>(W + (j + 1) * DP);
+                float z0 = -bb[j], z1 = -bb[j + 1], z0b = 0.f, z1b = 0.f;
 #pragma unroll
                 for (int i4 = 0; i4 < DP / 4; ++i4) {
-                    const float4 v = *reinterpret_cast<const float4*>(sx + pp * SX + 4 * i4);
-                    xr[4 * i4] = v.x; xr[4 * i4 + 1] = v.y; xr[4 * i4 + 2] = v.z; xr[4 * i4 + 3] = v.w;
+                    const float4 a = w0[i4], c = w1[i4];
+                    z0 = fmaf(a.x, xr[4 * i4 + 0], z0);
+                    z1 = fmaf(c.x, xr[4 * i4 + 0], z1);
+                    z0b = fmaf(a.y, xr[4 * i4 + 1], z0b);
+                    z1b = fmaf(c.y, xr[4 * i4 + 1], z1b);
+                    z0 = fmaf(a.z, xr[4 * i4 + 2], z0);
+                    z1 = fmaf(c.z, xr[4 * i4 + 2], z1);
+                    z0b = fmaf(a.w, xr[4 * i4 + 3], z0b);
+                    z1b = fmaf(c.w, xr[4 * i4 + 3], z1b);
                 }
-                float q0 = 0.f, q1 = 0.f;
-#pragma unroll 2
-                for (int j = 0; j < DP; j += 2) {
-                    const float4* w0 = reinterpret_cast<const float4*>(W + j * DP);
-                    const float4* w1 = reinterpret_cast<const float4*>(W + (j + 1) * DP);
-                    float z0 = -bb[j], z1 = -bb[j + 1], z0b = 0.f, z1b = 0.f;
-#pragma unroll
-                    for (int i4 = 0; i4 < DP / 4; ++i4) {
-                        const float4 a = w0[i4], c = w1[i4];
-                        z0 = fmaf(a.x, xr[4 * i4 + 0], z0);
-                        z1 = fmaf(c.x, xr[4 * i4 + 0], z1);
-                        z0b = fmaf(a.y, xr[4 * i4 + 1], z0b);
-                        z1b = fmaf(c.y, xr[4 * i4 + 1], z1b);
-                        z0 = fmaf(a.z, xr[4 * i4 + 2], z0);
-                        z1 = fmaf(c.z, xr[4 * i4 + 2], z1);
-                        z0b = fmaf(a.w, xr[4 * i4 + 3], z0b);
-                        z1b = fmaf(c.w, xr[4 * i4 + 3], z1b);
-                    }
-                    z0 += z0b;
-                    z1 += z1b;
-                    q0 = fmaf(z0, z0, q0);
-                    q1 = fmaf(z1, z1, q1);
-                }
-                sq[side * TP + pp] = q0 + q1;
-                __syncthreads();
-            } else {
-                if (tid < nt) {
-                    const float* xp = sx + tid * SX;
-                    float ql = 0.f, qr = 0.f;
-                    for (int j = 0; j < DP; ++j) {
-                        const float* wlp = sWl + j * DP;
-                        const float* wrp = sWr + j * DP;
-                        float zl = -sbl[j], zr = -sbr[j];
-#pragma unroll 8
-                        for (int i = 0; i < DP; ++i) {
-                            float xv = xp[i];
-                            zl = fmaf(wlp[i], xv, zl);
-                            zr = fmaf(wrp[i], xv, zr);
-                        }
-                        ql = fmaf(zl, zl, ql);
-                        qr = fmaf(zr, zr, qr);
-                    }
-                    sq[tid] = ql;
-                    sq[TP + tid] = qr;
-                }
+                z0 += z0b;
+                z1 += z1b;
+                q0 = fmaf(z0, z0, q0);
+                q1 = fmaf(z1, z1, q1);
             }
+            sq[side * TP + pp] = q0 + q1;
+            __syncthreads();
         }
         int sv = 0;
         if (tid < nt) {
@@ -1404,71 +1350,49 @@ __global__ void __launch_bounds__(256, (DP >= 128 ? 1 : 2)) k_gauss_sub_stats(
         }
         cnt_l += __syncthreads_count(sv == 1);
         cnt_r += __syncthreads_count(sv == 2);
-        if (PREFETCH && t0 + TP < len) load_tile(t0 + TP);
-        if constexpr (S::BLOCKED) {
-            if (grp < S::G) {
-                // two points per iteration: both points' loads issue before either's FMAs
-                auto acc = [&](int sv2, const float4 xi, const float4 xj) {
-                    const float vi[4] = {xi.x, xi.y, xi.z, xi.w};
-                    const float vj[4] = {xj.x, xj.y, xj.z, xj.w};
-                    if (sv2 == 1) {
+        if (t0 + TP < len) load_tile(t0 + TP);
+        if (grp < S::G) {
+            // two points per iteration: both points' loads issue before either's FMAs
+            auto acc = [&](int sv2, const float4 xi, const float4 xj) {
+                const float vi[4] = {xi.x, xi.y, xi.z, xi.w};
+                const float vj[4] = {xj.x, xj.y, xj.z, xj.w};
+                if (sv2 == 1) {
 #pragma unroll
-                        for (int a = 0; a < 4; ++a)
+                    for (int a = 0; a < 4; ++a)
 #pragma unroll
-                            for (int c = 0; c < 4; ++c) bf[0][4 * a + c] = fmaf(vi[a], vj[c], bf[0][4 * a + c]);
-                        if (diag) {
+                        for (int c = 0; c < 4; ++c) bf[0][4 * a + c] = fmaf(vi[a], vj[c], bf[0][4 * a + c]);
+                    if (diag) {
 #pragma unroll
-                            for (int a = 0; a < 4; ++a) sf[0][a] += vi[a];
-                        }
-                    } else if (sv2 == 2) {
-#pragma unroll
-                        for (int a = 0; a < 4; ++a)
-#pragma unroll
-                            for (int c = 0; c < 4; ++c) bf[1][4 * a + c] = fmaf(vi[a], vj[c], bf[1][4 * a + c]);
-                        if (diag) {
-#pragma unroll
-                            for (int a = 0; a < 4; ++a) sf[1][a] += vi[a];
-                        }
+                        for (int a = 0; a < 4; ++a) sf[0][a] += vi[a];
                     }
-                };
-                int run = 0;
-                for (int pp = grp; pp < nt; pp += 2 * S::G) {
-                    const int pq = pp + S::G;
-                    const int sa = ssub[pp];
-                    const int sb2 = pq < nt ? ssub[pq] : 0;
-                    if (has_blk) {
-                        const float* xa = sx + pp * SX;
-                        const float* xb = sx + (pq < nt ? pq : pp) * SX;
-                        const float4 xia = *reinterpret_cast<const float4*>(xa + 4 * bi);
-                        const float4 xja = *reinterpret_cast<const float4*>(xa + 4 * bj);
-                        const float4 xib = *reinterpret_cast<const float4*>(xb + 4 * bi);
-                        const float4 xjb = *reinterpret_cast<const float4*>(xb + 4 * bj);
-                        acc(sa, xia, xja);
-                        acc(sb2, xib, xjb);
-                    }
-                    run += ((sa == 1 || sa == 2) ? 1 : 0) + ((sb2 == 1 || sb2 == 2) ? 1 : 0);
-                    if (run >= 32) { flush(); run = 0; }   // FP32 runs of at most 33 points
-                }
-            }
-        } else {
-            for (int pp = 0; pp < nt; ++pp) {
-                const int sv2 = ssub[pp];
-                if (sv2 != 1 && sv2 != 2) continue;
-                const float* xp = sx + pp * SX;
-                const int slot = sv2 - 1;
+                } else if (sv2 == 2) {
 #pragma unroll
-                for (int m = 0; m < E; ++m) {
-                    int e = tid + 256 * m;
-                    if (e < T) {
-                        uint16_t pr = spair[e];
-                        int i = pr >> 8, j = pr & 0xff;
-                        if (slot == 0) accf[0][m] = fmaf(xp[i], xp[j], accf[0][m]);
-                        else accf[1][m] = fmaf(xp[i], xp[j], accf[1][m]);
+                    for (int a = 0; a < 4; ++a)
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) bf[1][4 * a + c] = fmaf(vi[a], vj[c], bf[1][4 * a + c]);
+                    if (diag) {
+#pragma unroll
+                        for (int a = 0; a < 4; ++a) sf[1][a] += vi[a];
                     }
                 }
-                if (slot == 0 && tid < DP) sumf += xp[tid];
-                if (slot == 1 && tid >= DP && tid < 2 * DP) sumf += xp[tid - DP];
-                if ((pp & 31) == 31) flush();
+            };
+            int run = 0;
+            for (int pp = grp; pp < nt; pp += 2 * S::G) {
+                const int pq = pp + S::G;
+                const int sa = ssub[pp];
+                const int sb2 = pq < nt ? ssub[pq] : 0;
+                if (has_blk) {
+                    const float* xa = sx + pp * SX;
+                    const float* xb = sx + (pq < nt ? pq : pp) * SX;
+                    const float4 xia = *reinterpret_cast<const float4*>(xa + 4 * bi);
+                    const float4 xja = *reinterpret_cast<const float4*>(xa + 4 * bj);
+                    const float4 xib = *reinterpret_cast<const float4*>(xb + 4 * bi);
+                    const float4 xjb = *reinterpret_cast<const float4*>(xb + 4 * bj);
+                    acc(sa, xia, xja);
+                    acc(sb2, xib, xjb);
+                }
+                run += ((sa == 1 || sa == 2) ? 1 : 0) + ((sb2 == 1 || sb2 == 2) ? 1 : 0);
+                if (run >= 32) { flush(); run = 0; }   // FP32 runs of at most 33 points
             }
         }
         flush();
@@ -1476,39 +1400,222 @@ __global__ void __launch_bounds__(256, (DP >= 128 ? 1 : 2)) k_gauss_sub_stats(
     double* pl = part + (size_t)ch * 2 * SL;
     double* pr = pl + SL;
     if (tid == 0) { pl[0] = (double)cnt_l; pr[0] = (double)cnt_r; }
-    if constexpr (S::BLOCKED) {
-        __syncthreads();
-        // sum the groups' FP64 totals; thread b < NBLK writes block b
-        if (tid < S::NBLK) {
-            int ri = 0, rem = tid;
-            while (rem >= S::NB - ri) { rem -= S::NB - ri; ++ri; }
-            const int rj = ri + rem;
+    __syncthreads();
+    // sum the groups' FP64 totals; thread b < NBLK writes block b
+    if (tid < S::NBLK) {
+        int ri = 0, rem = tid;
+        while (rem >= S::NB - ri) { rem -= S::NB - ri; ++ri; }
+        const int rj = ri + rem;
 #pragma unroll 1
-            for (int s2 = 0; s2 < 2; ++s2) {
-                double* po = s2 ? pr : pl;
-                for (int m = 0; m < 16; ++m) {
-                    const int i = 4 * ri + (m >> 2), j = 4 * rj + (m & 3);
-                    if (i > j) continue;
-                    double v = 0.0;
-                    for (int g = 0; g < S::G; ++g) v += stot[(16 * s2 + m) * S::NTOT + g * S::NBLK + tid];
-                    po[1 + DP + tri_index(DP, i, j)] = v;
-                }
+        for (int s2 = 0; s2 < 2; ++s2) {
+            double* po = s2 ? pr : pl;
+            for (int m = 0; m < 16; ++m) {
+                const int i = 4 * ri + (m >> 2), j = 4 * rj + (m & 3);
+                if (i > j) continue;
+                double v = 0.0;
+                for (int g = 0; g < S::G; ++g) v += stot[(16 * s2 + m) * S::NTOT + g * S::NBLK + tid];
+                po[1 + DP + tri_index(DP, i, j)] = v;
             }
         }
-        for (int e = tid; e < 2 * DP; e += 256) {
-            double v = 0.0;
-            for (int g = 0; g < S::G; ++g) v += ssum[g * 2 * DP + e];
-            (e < DP ? pl : pr)[1 + (e % DP)] = v;
-        }
-    } else {
-        if (tid < DP) pl[1 + tid] = sumd;
-        else if (tid < 2 * DP) pr[1 + tid - DP] = sumd;
+    }
+    for (int e = tid; e < 2 * DP; e += 256) {
+        double v = 0.0;
+        for (int g = 0; g < S::G; ++g) v += ssum[g * 2 * DP + e];
+        (e < DP ? pl : pr)[1 + (e % DP)] = v;
+    }
+}
+
+// Dp = 128: the sub-label draws and the statistics as two kernels.
+//
+// Draws: one block per tile of 128 points of a chunk; warps 0-3 evaluate the l factor, warps 4-7 the r factor, a thread
+// per point with x - s in registers.  The factors are transposed in shared memory, so that four outputs come
+// with one 16-byte read and two go through one packed multiply-add; each z_j stays one chain over the features, and
+// |z|^2 one chain over j.  Bound: those reads.
+constexpr int kWideLD = 132;   // shared row stride of 128 floats (16-byte rows)
+__global__ void __launch_bounds__(256, 1) k_gauss_sub_draw_wide(
+    const float* __restrict__ x, const int32_t* __restrict__ perm, const int32_t* __restrict__ chunk,
+    const int32_t* __restrict__ nchunks, const float* __restrict__ Wt, const float* __restrict__ bvec,
+    const float* __restrict__ cvec, const float* __restrict__ lrw, const float* __restrict__ muv, RngArgs rng,
+    int32_t* __restrict__ sub, float* __restrict__ r_out, const uint8_t* __restrict__ mask)
+{
+    constexpr int DP = 128, TP = 128;
+    extern __shared__ __align__(16) unsigned char smem[];
+    float* sW = reinterpret_cast<float*>(smem);       // [2][i][kWideLD]: W(i, j), j contiguous
+    float* sb = sW + 2 * DP * kWideLD;                // [2][DP] b - W^T s
+    float* ss = sb + 2 * DP;                          // [DP] s, the cluster's mean parameter
+    float* sq = ss + DP;                              // [2][TP]
+    const int ch = blockIdx.x, t0 = (int)blockIdx.y * TP;
+    if (ch >= *nchunks) return;
+    const int k = chunk[3 * ch], start = chunk[3 * ch + 1], len = chunk[3 * ch + 2];
+    if (t0 >= len || (mask && !mask[k])) return;
+    const int tid = threadIdx.x, side = tid >> 7, pp = tid & 127;
+    const int64_t pt = perm[start + min(t0 + pp, len - 1)];
+    for (int e = tid; e < 2 * DP * DP / 4; e += 256) {
+        const int sd = e / (DP * DP / 4), j = e / (DP / 4) % DP, i4 = e % (DP / 4);
+        const float4 v = reinterpret_cast<const float4*>(Wt + (size_t)(3 * k + 1 + sd) * DP * DP)[j * (DP / 4) + i4];
+        float* dst = sW + (size_t)(sd * DP + 4 * i4) * kWideLD + j;
+        dst[0] = v.x;
+        dst[kWideLD] = v.y;
+        dst[2 * kWideLD] = v.z;
+        dst[3 * kWideLD] = v.w;
+    }
+    if (tid < DP) ss[tid] = muv[(size_t)(3 * k) * DP + tid];
+    __syncthreads();
+    {
+        float acc = 0.f;
+        for (int i = 0; i < DP; ++i) acc = fmaf(sW[(side * DP + i) * kWideLD + pp], ss[i], acc);
+        sb[side * DP + pp] = bvec[(size_t)(3 * k + 1 + side) * DP + pp] - acc;
+    }
+    float xr[DP];
 #pragma unroll
-        for (int m = 0; m < E; ++m) {
-            int e = tid + 256 * m;
-            if (e < T) { pl[1 + DP + e] = accd[0][m]; pr[1 + DP + e] = accd[1][m]; }
+    for (int i4 = 0; i4 < DP / 4; ++i4) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(x + pt * DP) + i4);
+        const float4 s4 = *reinterpret_cast<const float4*>(ss + 4 * i4);
+        xr[4 * i4] = v.x - s4.x;
+        xr[4 * i4 + 1] = v.y - s4.y;
+        xr[4 * i4 + 2] = v.z - s4.z;
+        xr[4 * i4 + 3] = v.w - s4.w;
+    }
+    __syncthreads();
+    const float* Ws = sW + (size_t)side * DP * kWideLD;
+    float q = 0.f;
+#pragma unroll 1
+    for (int j0 = 0; j0 < DP; j0 += 16) {
+        uint64_t z[8];
+#pragma unroll
+        for (int m = 0; m < 8; ++m) z[m] = pack2(-sb[side * DP + j0 + 2 * m], -sb[side * DP + j0 + 2 * m + 1]);
+#pragma unroll
+        for (int i = 0; i < DP; ++i) {
+            const ulonglong2* w = reinterpret_cast<const ulonglong2*>(Ws + i * kWideLD + j0);
+            const uint64_t xi = pack2(xr[i], xr[i]);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                const ulonglong2 ww = w[m];
+                z[2 * m] = fma2(ww.x, xi, z[2 * m]);
+                z[2 * m + 1] = fma2(ww.y, xi, z[2 * m + 1]);
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            float a, b;
+            unpack2(z[m], a, b);
+            q = fmaf(a, a, q);
+            q = fmaf(b, b, q);
         }
     }
+    sq[side * TP + pp] = q;
+    __syncthreads();
+    if (tid < TP && t0 + tid < len) {
+        const float rl = cvec[3 * k + 1] - 0.5f * sq[tid], rr = cvec[3 * k + 2] - 0.5f * sq[TP + tid];
+        if (r_out) { r_out[2 * pt] = rl; r_out[2 * pt + 1] = rr; }
+        float u1, u2;
+        draw_uniform2(rng, pt, u1, u2);
+        sub[pt] = draw_sub_label(rl + lrw[2 * k], rr + lrw[2 * k + 1], u1, u2);
+    }
+}
+
+// Statistics (the sub-labels are given): a block per chunk and sub-cluster; each of 136 threads owns an 8 x 8 block of
+// the upper triangle (the diagonal ones the sums too) and adds the side's points of every window of 32 points in FP32,
+// two columns per packed multiply-add, then the window into FP64 totals in registers.  Bound: the multiply-adds (32 a
+// point and thread).  With the draws, N = 1e5, D = 100, K = 12: 2515 -> 640 us (one matrix entry at a time through a
+// pair table, 33 entries a thread, and the draws by one half of the threads before).
+__global__ void __launch_bounds__(160) k_gauss_stats_wide(
+    const float* __restrict__ x, const int32_t* __restrict__ perm, const int32_t* __restrict__ chunk,
+    const int32_t* __restrict__ nchunks, const float* __restrict__ muv, const int32_t* __restrict__ sub,
+    double* __restrict__ part, const uint8_t* __restrict__ mask)
+{
+    constexpr int DP = 128, T = tri(DP), SL = 1 + DP + T, NB = DP / 8, TP = 64;
+    __shared__ __align__(16) float sx[TP * kWideLD];
+    __shared__ __align__(16) float ss[DP];
+    __shared__ int32_t ssub[TP];
+    const int ch = blockIdx.x, slot = (int)blockIdx.y + 1;
+    if (ch >= *nchunks) return;
+    const int k = chunk[3 * ch], start = chunk[3 * ch + 1], len = chunk[3 * ch + 2];
+    if (mask && !mask[k]) return;
+    const int tid = threadIdx.x;
+    if (tid < DP) ss[tid] = muv[(size_t)(3 * k) * DP + tid];
+    int bi = 0, bj = 0;
+    const bool own = tid < NB * (NB + 1) / 2;
+    if (own) {
+        int rem = tid;
+        while (rem >= NB - bi) { rem -= NB - bi; ++bi; }
+        bj = bi + rem;
+    }
+    const bool diag = own && bi == bj;
+    uint64_t acc[8][4];
+    float sf[8];
+    double accd[64], sd[8];
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[a][c] = 0;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) accd[8 * a + c] = 0.0;
+        sf[a] = 0.f;
+        sd[a] = 0.0;
+    }
+    int cnt = 0;
+    for (int t0 = 0; t0 < len; t0 += TP) {
+        const int nt = min(TP, len - t0);
+        __syncthreads();
+        for (int e = tid; e < nt * (DP / 4); e += 160) {
+            const int row = e / (DP / 4), i4 = e % (DP / 4);
+            const float4 v = __ldg(reinterpret_cast<const float4*>(x + (size_t)__ldg(perm + start + t0 + row) * DP) + i4);
+            const float4 s4 = *reinterpret_cast<const float4*>(ss + 4 * i4);
+            *reinterpret_cast<float4*>(sx + row * kWideLD + 4 * i4) = make_float4(v.x - s4.x, v.y - s4.y, v.z - s4.z, v.w - s4.w);
+        }
+        int sv = 0;
+        if (tid < nt) ssub[tid] = sv = sub[perm[start + t0 + tid]];
+        cnt += __syncthreads_count(sv == slot);
+        if (!own) continue;
+        for (int w0 = 0; w0 < nt; w0 += 32) {
+            const int w1 = min(nt, w0 + 32);
+            for (int p = w0; p < w1; ++p) {
+                if (ssub[p] != slot) continue;
+                const float* xp = sx + p * kWideLD;
+                const float4 i0 = *reinterpret_cast<const float4*>(xp + 8 * bi), i1 = *reinterpret_cast<const float4*>(xp + 8 * bi + 4);
+                const ulonglong2 j0 = *reinterpret_cast<const ulonglong2*>(xp + 8 * bj), j1 = *reinterpret_cast<const ulonglong2*>(xp + 8 * bj + 4);
+                const float vi[8] = {i0.x, i0.y, i0.z, i0.w, i1.x, i1.y, i1.z, i1.w};
+#pragma unroll
+                for (int a = 0; a < 8; ++a) {
+                    const uint64_t xi = pack2(vi[a], vi[a]);
+                    acc[a][0] = fma2(xi, j0.x, acc[a][0]);
+                    acc[a][1] = fma2(xi, j0.y, acc[a][1]);
+                    acc[a][2] = fma2(xi, j1.x, acc[a][2]);
+                    acc[a][3] = fma2(xi, j1.y, acc[a][3]);
+                }
+                if (diag)
+#pragma unroll
+                    for (int a = 0; a < 8; ++a) sf[a] += vi[a];
+            }
+#pragma unroll
+            for (int a = 0; a < 8; ++a) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    float u, v;
+                    unpack2(acc[a][c], u, v);
+                    accd[8 * a + 2 * c] += (double)u;
+                    accd[8 * a + 2 * c + 1] += (double)v;
+                    acc[a][c] = 0;
+                }
+                sd[a] += (double)sf[a];
+                sf[a] = 0.f;
+            }
+        }
+    }
+    double* po = part + ((size_t)ch * 2 + (slot - 1)) * SL;
+    if (tid == 0) po[0] = (double)cnt;
+    if (!own) return;
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const int i = 8 * bi + a, j = 8 * bj + c;
+            if (i <= j) po[1 + DP + tri_index(DP, i, j)] = accd[8 * a + c];
+        }
+    if (diag)
+#pragma unroll
+        for (int a = 0; a < 8; ++a) po[1 + 8 * bi + a] = sd[a];
 }
 
 // Statistics only (the sub-labels are given), DP <= 64: one pass per sub-cluster over the
@@ -1902,6 +2009,22 @@ static dpmm_status launch_mult_sub_stats_t(dpmm_ctx* c, RngArgs r, float* d_rout
     return DPMM_OK;
 }
 
+static dpmm_status launch_gauss_sub_stats_wide(dpmm_ctx* c, int draw, RngArgs r, float* d_rout, const uint8_t* d_mask)
+{
+    if (draw) {
+        constexpr size_t sm = sizeof(float) * (2 * 128 * kWideLD + 3 * 128 + 2 * 128);
+        DPMM_CUDA_TRY(cudaFuncSetAttribute(k_gauss_sub_draw_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        const dim3 grid((unsigned)c->max_chunks, (unsigned)((c->chunk_len + 127) / 128));
+        k_gauss_sub_draw_wide<<<grid, 256, sm, c->stream>>>(c->d_x, c->d_perm, c->d_chunk, c->d_nchunks, c->d_Wt, c->d_b, c->d_c,
+                                                            c->d_lrw, c->d_mu, r, c->d_sub, d_rout, d_mask);
+        DPMM_LAUNCHED();
+    }
+    k_gauss_stats_wide<<<dim3((unsigned)c->max_chunks, 2), 160, 0, c->stream>>>(c->d_x, c->d_perm, c->d_chunk, c->d_nchunks,
+                                                                               c->d_mu, c->d_sub, c->d_part, d_mask);
+    DPMM_LAUNCHED();
+    return DPMM_OK;
+}
+
 template <int DP>
 static dpmm_status launch_gauss_sub_stats_t(dpmm_ctx* c, int draw, RngArgs r, float* d_rout, const uint8_t* d_mask)
 {
@@ -1951,7 +2074,7 @@ dpmm_status launch_sub_labels_and_stats(dpmm_ctx* c, int K, const float* d_u, fl
             case 16: DPMM_TRY(launch_gauss_sub_stats_t<16>(c, draw, r, d_rout, d_mask)); break;
             case 32: DPMM_TRY(launch_gauss_sub_stats_t<32>(c, draw, r, d_rout, d_mask)); break;
             case 64: DPMM_TRY(launch_gauss_sub_stats_t<64>(c, draw, r, d_rout, d_mask)); break;
-            case 128: DPMM_TRY(launch_gauss_sub_stats_t<128>(c, draw, r, d_rout, d_mask)); break;
+            case 128: DPMM_TRY(launch_gauss_sub_stats_wide(c, draw, r, d_rout, d_mask)); break;
             default: return fail(DPMM_ERR_INVALID_ARG, "unsupported padded dimension");
         }
     } else {
