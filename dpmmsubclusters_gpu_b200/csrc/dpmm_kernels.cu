@@ -142,9 +142,32 @@ __device__ __forceinline__ int draw_from_r(float* sr, int p, int K, int final_, 
 // Gaussian label phase, FP32 SIMT: one thread per point, x in registers, each cluster's
 // precision factor (transposed) broadcast from shared memory.
 //   z_j = sum_i W(i,j) x_i - b_j,   r_k = c_k - 0.5 * sum_j z_j^2
-// r = c - 0.5 |W^T x - b|^2 for one point (x in registers, two features to a 64-bit pair) and one cluster whose
-// transposed factor (Wt[j][i] = W(i, j)) and b are staged in shared memory.  z_j is the sum of an even-feature and an
-// odd-feature chain, one packed multiply-add for both.
+// z_j and z_{j+1} of one point (x in registers, two features to a 64-bit pair) and one transposed factor (Wt[j][i] =
+// W(i, j), row j at w); b at bj.  z_j is the sum of an even-feature and an odd-feature chain, one packed multiply-add
+// for both.
+template <int DP>
+__device__ __forceinline__ void gauss_z_pair(const float* __restrict__ w, const float* __restrict__ bj,
+                                             const uint64_t (&x2)[DP / 2], float& z0, float& z1)
+{
+    const ulonglong2* w0 = reinterpret_cast<const ulonglong2*>(w);
+    const ulonglong2* w1 = reinterpret_cast<const ulonglong2*>(w + DP);
+    uint64_t a0 = pack2(-bj[0], 0.f), a1 = pack2(-bj[1], 0.f);
+#pragma unroll
+    for (int i4 = 0; i4 < DP / 4; ++i4) {
+        const ulonglong2 a = w0[i4], b = w1[i4];
+        a0 = fma2(a.x, x2[2 * i4], a0);
+        a1 = fma2(b.x, x2[2 * i4], a1);
+        a0 = fma2(a.y, x2[2 * i4 + 1], a0);
+        a1 = fma2(b.y, x2[2 * i4 + 1], a1);
+    }
+    float e, o;
+    unpack2(a0, e, o);
+    z0 = e + o;
+    unpack2(a1, e, o);
+    z1 = e + o;
+}
+
+// r = c - 0.5 |W^T x - b|^2 for one point and one cluster whose transposed factor and b are staged in shared memory
 template <int DP>
 __device__ __forceinline__ float gauss_r_pairs(const float* __restrict__ sW, const float* __restrict__ sbv,
                                                const uint64_t (&x2)[DP / 2], float c)
@@ -152,24 +175,10 @@ __device__ __forceinline__ float gauss_r_pairs(const float* __restrict__ sW, con
     float q = 0.f;
 #pragma unroll 2
     for (int j = 0; j < DP; j += 2) {
-        const ulonglong2* w0 = reinterpret_cast<const ulonglong2*>(sW + j * DP);
-        const ulonglong2* w1 = reinterpret_cast<const ulonglong2*>(sW + (j + 1) * DP);
-        uint64_t z0 = pack2(-sbv[j], 0.f), z1 = pack2(-sbv[j + 1], 0.f);
-#pragma unroll
-        for (int i4 = 0; i4 < DP / 4; ++i4) {
-            const ulonglong2 a = w0[i4], b = w1[i4];
-            z0 = fma2(a.x, x2[2 * i4], z0);
-            z1 = fma2(b.x, x2[2 * i4], z1);
-            z0 = fma2(a.y, x2[2 * i4 + 1], z0);
-            z1 = fma2(b.y, x2[2 * i4 + 1], z1);
-        }
-        float e, o;
-        unpack2(z0, e, o);
-        e += o;
-        q = fmaf(e, e, q);
-        unpack2(z1, e, o);
-        e += o;
-        q = fmaf(e, e, q);
+        float z0, z1;
+        gauss_z_pair<DP>(sW + j * DP, sbv + j, x2, z0, z1);
+        q = fmaf(z0, z0, q);
+        q = fmaf(z1, z1, q);
     }
     return c - 0.5f * q;
 }
@@ -1127,11 +1136,16 @@ dpmm_status build_permutation(dpmm_ctx* c, int K)
 //
 // DP <= 64, 128 points per tile (the two kernels below take DP = 128):
 //   draw  - two threads per point, one per side: warps 0-3 evaluate the l factor, warps 4-7 the r
-//           factor, x in registers, factor rows broadcast from shared memory as float4;
-//   stats - each thread of a warp-aligned group owns one 4 x 4 block of the upper triangle and
-//           does 16 FMAs per point from two float4 loads; G groups take every G-th point of the
-//           tile; FP64 totals per thread live in shared memory and are summed over the groups at
-//           the end.
+//           factor, x in registers, factor rows broadcast from shared memory, two features to a
+//           packed multiply-add;
+//   stats - G warp-aligned groups take every G-th point of the tile; each thread of a group owns one
+//           4 x 4 block of the upper triangle, or (DP <= 16, where a warp has 1 to 10 blocks) one or
+//           two rows of it for one or both sides, and adds the point's products two columns at a time.
+//           The FP64 totals (in shared memory, or in registers at DP <= 16) are summed over the groups
+//           at the end.
+// Bound: the draws' reads of the factors (DP >= 32), else barriers and the draws' special functions.  A launch at
+// N = 1e6, D = 7, K = 30 took 154 us with a 4 x 4 block per thread at every width (3 of 32 lanes busy) and takes 57;
+// N = 2000, D = 2: 30 -> 11.5 us; batches at D = 16 and 64: 35 -> 27 and 239 -> 222 us.
 
 template <int DP>
 struct SubStatsShape {
@@ -1140,8 +1154,14 @@ struct SubStatsShape {
     static constexpr int NB = DP / 4;
     static constexpr int NBLK = NB * (NB + 1) / 2;                   // 4 x 4 blocks of the triangle
     static constexpr int GS = (NBLK + 31) / 32 * 32;                 // threads per group (whole warps)
-    static constexpr int G = 256 / GS;                 // groups
+    static constexpr int G = 256 / GS;                               // groups
     static constexpr int NTOT = G * NBLK;                            // owners of FP64 totals
+    // DP <= 16: a group is one warp with few blocks; they are cut into row parts (and sides) over its lanes
+    static constexpr bool ROWS = DP <= 16;
+    static constexpr int RW = DP <= 8 ? 1 : DP == 16 ? 2 : 4;                    // rows of a block per lane
+    static constexpr int NS = DP <= 8 ? 1 : 2;                       // sides per lane
+    static constexpr int PARTS = (4 / RW) * (2 / NS);                // lanes per block
+    static_assert(!ROWS || NBLK * PARTS <= 32, "a group's parts fit its warp");
     // shared layout in bytes
     static constexpr size_t off_wl = 0;
     static constexpr size_t off_wr = off_wl + sizeof(float) * DP * DP;
@@ -1158,7 +1178,7 @@ struct SubStatsShape {
 };
 
 template <int DP>
-__global__ void __launch_bounds__(256, 2) k_gauss_sub_stats(
+__global__ void __launch_bounds__(256, (DP <= 8 ? 4 : DP == 16 ? 3 : 2)) k_gauss_sub_stats(
     const float* __restrict__ x, const int32_t* __restrict__ perm, const int32_t* __restrict__ chunk,
     const int32_t* __restrict__ nchunks, const float* __restrict__ Wt, const float* __restrict__ bvec,
     const float* __restrict__ cvec, const float* __restrict__ lrw, const float* __restrict__ muv, int draw,
@@ -1215,8 +1235,10 @@ __global__ void __launch_bounds__(256, 2) k_gauss_sub_stats(
     const float cl = draw ? cvec[3 * k + 1] : 0.f, cr = draw ? cvec[3 * k + 2] : 0.f;
     const float wl = draw ? lrw[2 * k] : 0.f, wr = draw ? lrw[2 * k + 1] : 0.f;
 
-    // this thread's group, 4 x 4 block (bi <= bj) and FP64 total column
-    const int grp = tid / S::GS, tb = tid % S::GS;
+    // this thread's group and 4 x 4 block (bi <= bj); of that the rows from row0 of the sides from side0 (DP <= 16),
+    // else all of it and a column of FP64 totals
+    const int grp = tid / S::GS, tb = (tid % S::GS) / S::PARTS, pc = tid % S::GS % S::PARTS;
+    const int row0 = pc % (4 / S::RW) * S::RW, side0 = pc / (4 / S::RW);
     const bool has_blk = grp < S::G && tb < S::NBLK;
     int bi = 0, bj = 0;
     if (has_blk) {
@@ -1226,39 +1248,46 @@ __global__ void __launch_bounds__(256, 2) k_gauss_sub_stats(
     }
     const bool diag = has_blk && bi == bj;
     const int tcol = grp * S::NBLK + tb;
-    if (has_blk)
-        for (int m = 0; m < 32; ++m) stot[m * S::NTOT + tcol] = 0.0;
-    for (int e = tid; e < S::G * 2 * DP; e += 256) ssum[e] = 0.0;
-    float bf[2][16];
-    float sf[2][4];
-#pragma unroll
-    for (int s2 = 0; s2 < 2; ++s2) {
-#pragma unroll
-        for (int m = 0; m < 16; ++m) bf[s2][m] = 0.f;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) sf[s2][m] = 0.f;
+    if constexpr (!S::ROWS) {
+        if (has_blk)
+            for (int m = 0; m < 32; ++m) stot[m * S::NTOT + tcol] = 0.0;
+        for (int e = tid; e < S::G * 2 * DP; e += 256) ssum[e] = 0.0;
     }
+    uint64_t bf[S::NS][S::RW][2];       // FP32 runs: [side][row][pair of columns]
+    float sf[S::NS][S::RW];
+    double td[S::NS][S::RW][5];         // DP <= 16: their FP64 totals, the sum last
+#pragma unroll
+    for (int s2 = 0; s2 < S::NS; ++s2)
+#pragma unroll
+        for (int a = 0; a < S::RW; ++a) {
+            bf[s2][a][0] = bf[s2][a][1] = 0;
+            sf[s2][a] = 0.f;
+#pragma unroll
+            for (int c = 0; c < 5; ++c) td[s2][a][c] = 0.0;
+        }
     int cnt_l = 0, cnt_r = 0;
 
     auto flush = [&]() {
-        if (has_blk) {
+        if (!has_blk) return;
 #pragma unroll
-            for (int s2 = 0; s2 < 2; ++s2)
+        for (int s2 = 0; s2 < S::NS; ++s2)
 #pragma unroll
-                for (int m = 0; m < 16; ++m) {
-                    stot[(16 * s2 + m) * S::NTOT + tcol] += (double)bf[s2][m];
-                    bf[s2][m] = 0.f;
+            for (int a = 0; a < S::RW; ++a) {
+                float v[4];
+                unpack2(bf[s2][a][0], v[0], v[1]);
+                unpack2(bf[s2][a][1], v[2], v[3]);
+                bf[s2][a][0] = bf[s2][a][1] = 0;
+                if constexpr (S::ROWS) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) td[s2][a][c] += (double)v[c];
+                    td[s2][a][4] += (double)sf[s2][a];
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) stot[(16 * s2 + 4 * a + c) * S::NTOT + tcol] += (double)v[c];
+                    if (diag) ssum[(grp * 2 + s2) * DP + 4 * bi + a] += (double)sf[s2][a];
                 }
-            if (diag) {
-#pragma unroll
-                for (int s2 = 0; s2 < 2; ++s2)
-#pragma unroll
-                    for (int a = 0; a < 4; ++a) {
-                        ssum[(grp * 2 + s2) * DP + 4 * bi + a] += (double)sf[s2][a];
-                        sf[s2][a] = 0.f;
-                    }
+                sf[s2][a] = 0.f;
             }
-        }
     };
 
     // tile staging: each thread holds NPF float4 of the next tile in registers, loaded while the
@@ -1298,32 +1327,18 @@ __global__ void __launch_bounds__(256, 2) k_gauss_sub_stats(
             const int side = tid >> 7, pp = tid & 127;
             const float* W = side ? sWr : sWl;
             const float* bb = side ? sbr : sbl;
-            float xr[DP];
+            uint64_t x2[DP / 2];
 #pragma unroll
             for (int i4 = 0; i4 < DP / 4; ++i4) {
-                const float4 v = *reinterpret_cast<const float4*>(sx + pp * SX + 4 * i4);
-                xr[4 * i4] = v.x; xr[4 * i4 + 1] = v.y; xr[4 * i4 + 2] = v.z; xr[4 * i4 + 3] = v.w;
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(sx + pp * SX + 4 * i4);
+                x2[2 * i4] = v.x;
+                x2[2 * i4 + 1] = v.y;
             }
             float q0 = 0.f, q1 = 0.f;
 #pragma unroll 2
             for (int j = 0; j < DP; j += 2) {
-                const float4* w0 = reinterpret_cast<const float4*>(W + j * DP);
-                const float4* w1 = reinterpret_cast<const float4*>(W + (j + 1) * DP);
-                float z0 = -bb[j], z1 = -bb[j + 1], z0b = 0.f, z1b = 0.f;
-#pragma unroll
-                for (int i4 = 0; i4 < DP / 4; ++i4) {
-                    const float4 a = w0[i4], c = w1[i4];
-                    z0 = fmaf(a.x, xr[4 * i4 + 0], z0);
-                    z1 = fmaf(c.x, xr[4 * i4 + 0], z1);
-                    z0b = fmaf(a.y, xr[4 * i4 + 1], z0b);
-                    z1b = fmaf(c.y, xr[4 * i4 + 1], z1b);
-                    z0 = fmaf(a.z, xr[4 * i4 + 2], z0);
-                    z1 = fmaf(c.z, xr[4 * i4 + 2], z1);
-                    z0b = fmaf(a.w, xr[4 * i4 + 3], z0b);
-                    z1b = fmaf(c.w, xr[4 * i4 + 3], z1b);
-                }
-                z0 += z0b;
-                z1 += z1b;
+                float z0, z1;
+                gauss_z_pair<DP>(W + j * DP, bb + j, x2, z0, z1);
                 q0 = fmaf(z0, z0, q0);
                 q1 = fmaf(z1, z1, q1);
             }
@@ -1352,47 +1367,60 @@ __global__ void __launch_bounds__(256, 2) k_gauss_sub_stats(
         cnt_r += __syncthreads_count(sv == 2);
         if (t0 + TP < len) load_tile(t0 + TP);
         if (grp < S::G) {
-            // two points per iteration: both points' loads issue before either's FMAs
-            auto acc = [&](int sv2, const float4 xi, const float4 xj) {
-                const float vi[4] = {xi.x, xi.y, xi.z, xi.w};
-                const float vj[4] = {xj.x, xj.y, xj.z, xj.w};
-                if (sv2 == 1) {
+            auto acc = [&](int sv2, const float (&xi)[S::RW], const ulonglong2 xj) {
 #pragma unroll
-                    for (int a = 0; a < 4; ++a)
+                for (int s2 = 0; s2 < S::NS; ++s2)
+                    if (sv2 == side0 + s2 + 1)
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) bf[0][4 * a + c] = fmaf(vi[a], vj[c], bf[0][4 * a + c]);
-                    if (diag) {
-#pragma unroll
-                        for (int a = 0; a < 4; ++a) sf[0][a] += vi[a];
-                    }
-                } else if (sv2 == 2) {
-#pragma unroll
-                    for (int a = 0; a < 4; ++a)
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) bf[1][4 * a + c] = fmaf(vi[a], vj[c], bf[1][4 * a + c]);
-                    if (diag) {
-#pragma unroll
-                        for (int a = 0; a < 4; ++a) sf[1][a] += vi[a];
-                    }
+                        for (int a = 0; a < S::RW; ++a) {
+                            const uint64_t xa = pack2(xi[a], xi[a]);
+                            bf[s2][a][0] = fma2(xa, xj.x, bf[s2][a][0]);
+                            bf[s2][a][1] = fma2(xa, xj.y, bf[s2][a][1]);
+                            sf[s2][a] += xi[a];
+                        }
+            };
+            auto rows = [&](const float* xp, float (&xi)[S::RW]) {
+                if constexpr (S::RW == 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(xp + 4 * bi);
+                    xi[0] = v.x, xi[1] = v.y, xi[2] = v.z, xi[3] = v.w;
+                } else if constexpr (S::RW == 2) {
+                    const float2 v = *reinterpret_cast<const float2*>(xp + 4 * bi + row0);
+                    xi[0] = v.x, xi[1] = v.y;
+                } else {
+                    xi[0] = xp[4 * bi + row0];
                 }
             };
-            int run = 0;
-            for (int pp = grp; pp < nt; pp += 2 * S::G) {
-                const int pq = pp + S::G;
-                const int sa = ssub[pp];
-                const int sb2 = pq < nt ? ssub[pq] : 0;
-                if (has_blk) {
-                    const float* xa = sx + pp * SX;
-                    const float* xb = sx + (pq < nt ? pq : pp) * SX;
-                    const float4 xia = *reinterpret_cast<const float4*>(xa + 4 * bi);
-                    const float4 xja = *reinterpret_cast<const float4*>(xa + 4 * bj);
-                    const float4 xib = *reinterpret_cast<const float4*>(xb + 4 * bi);
-                    const float4 xjb = *reinterpret_cast<const float4*>(xb + 4 * bj);
-                    acc(sa, xia, xja);
-                    acc(sb2, xib, xjb);
+            if constexpr (S::ROWS) {
+                // a group has at most 16 points of the tile: one run
+                if (has_blk)
+#pragma unroll 4
+                    for (int pp = grp; pp < nt; pp += S::G) {
+                        const float* xp = sx + pp * SX;
+                        float xi[S::RW];
+                        rows(xp, xi);
+                        acc(ssub[pp], xi, *reinterpret_cast<const ulonglong2*>(xp + 4 * bj));
+                    }
+            } else {
+                // two points per iteration: both points' loads issue before either's multiply-adds
+                int run = 0;
+                for (int pp = grp; pp < nt; pp += 2 * S::G) {
+                    const int pq = pp + S::G;
+                    const int sa = ssub[pp];
+                    const int sb2 = pq < nt ? ssub[pq] : 0;
+                    if (has_blk) {
+                        const float* xa = sx + pp * SX;
+                        const float* xb = sx + (pq < nt ? pq : pp) * SX;
+                        float xia[S::RW], xib[S::RW];
+                        rows(xa, xia);
+                        rows(xb, xib);
+                        const ulonglong2 xja = *reinterpret_cast<const ulonglong2*>(xa + 4 * bj);
+                        const ulonglong2 xjb = *reinterpret_cast<const ulonglong2*>(xb + 4 * bj);
+                        acc(sa, xia, xja);
+                        acc(sb2, xib, xjb);
+                    }
+                    run += ((sa == 1 || sa == 2) ? 1 : 0) + ((sb2 == 1 || sb2 == 2) ? 1 : 0);
+                    if (run >= 32) { flush(); run = 0; }   // FP32 runs of at most 33 points
                 }
-                run += ((sa == 1 || sa == 2) ? 1 : 0) + ((sb2 == 1 || sb2 == 2) ? 1 : 0);
-                if (run >= 32) { flush(); run = 0; }   // FP32 runs of at most 33 points
             }
         }
         flush();
@@ -1400,23 +1428,29 @@ __global__ void __launch_bounds__(256, 2) k_gauss_sub_stats(
     double* pl = part + (size_t)ch * 2 * SL;
     double* pr = pl + SL;
     if (tid == 0) { pl[0] = (double)cnt_l; pr[0] = (double)cnt_r; }
+    if constexpr (S::ROWS) {
+        if (has_blk)
+#pragma unroll
+            for (int s2 = 0; s2 < S::NS; ++s2)
+#pragma unroll
+                for (int a = 0; a < S::RW; ++a) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        stot[(16 * (side0 + s2) + 4 * (row0 + a) + c) * S::NTOT + tcol] = td[s2][a][c];
+                    if (diag) ssum[(grp * 2 + side0 + s2) * DP + 4 * bi + row0 + a] = td[s2][a][4];
+                }
+    }
     __syncthreads();
-    // sum the groups' FP64 totals; thread b < NBLK writes block b
-    if (tid < S::NBLK) {
-        int ri = 0, rem = tid;
+    // sum the groups' FP64 totals, a thread per entry
+    for (int e = tid; e < 32 * S::NBLK; e += 256) {
+        const int m = e / S::NBLK % 16, b = e % S::NBLK;
+        int ri = 0, rem = b;
         while (rem >= S::NB - ri) { rem -= S::NB - ri; ++ri; }
-        const int rj = ri + rem;
-#pragma unroll 1
-        for (int s2 = 0; s2 < 2; ++s2) {
-            double* po = s2 ? pr : pl;
-            for (int m = 0; m < 16; ++m) {
-                const int i = 4 * ri + (m >> 2), j = 4 * rj + (m & 3);
-                if (i > j) continue;
-                double v = 0.0;
-                for (int g = 0; g < S::G; ++g) v += stot[(16 * s2 + m) * S::NTOT + g * S::NBLK + tid];
-                po[1 + DP + tri_index(DP, i, j)] = v;
-            }
-        }
+        const int i = 4 * ri + (m >> 2), j = 4 * (ri + rem) + (m & 3);
+        if (i > j) continue;
+        double v = 0.0;
+        for (int g = 0; g < S::G; ++g) v += stot[(e / S::NBLK) * S::NTOT + g * S::NBLK + b];
+        (e < 16 * S::NBLK ? pl : pr)[1 + DP + tri_index(DP, i, j)] = v;
     }
     for (int e = tid; e < 2 * DP; e += 256) {
         double v = 0.0;
