@@ -144,16 +144,16 @@ __device__ __forceinline__ int draw_from_r(float* sr, int p, int K, int final_, 
 //   z_j = sum_i W(i,j) x_i - b_j,   r_k = c_k - 0.5 * sum_j z_j^2
 // z_j and z_{j+1} of one point (x in registers, two features to a 64-bit pair) and one transposed factor (Wt[j][i] =
 // W(i, j), row j at w); b at bj.  z_j is the sum of an even-feature and an odd-feature chain, one packed multiply-add
-// for both.
-template <int DP>
+// for both.  E: the features and rows that are used and staged (see gauss_labels_tile).
+template <int E>
 __device__ __forceinline__ void gauss_z_pair(const float* __restrict__ w, const float* __restrict__ bj,
-                                             const uint64_t (&x2)[DP / 2], float& z0, float& z1)
+                                             const uint64_t (&x2)[E / 2], float& z0, float& z1)
 {
     const ulonglong2* w0 = reinterpret_cast<const ulonglong2*>(w);
-    const ulonglong2* w1 = reinterpret_cast<const ulonglong2*>(w + DP);
+    const ulonglong2* w1 = reinterpret_cast<const ulonglong2*>(w + E);
     uint64_t a0 = pack2(-bj[0], 0.f), a1 = pack2(-bj[1], 0.f);
 #pragma unroll
-    for (int i4 = 0; i4 < DP / 4; ++i4) {
+    for (int i4 = 0; i4 < E / 4; ++i4) {
         const ulonglong2 a = w0[i4], b = w1[i4];
         a0 = fma2(a.x, x2[2 * i4], a0);
         a1 = fma2(b.x, x2[2 * i4], a1);
@@ -168,15 +168,15 @@ __device__ __forceinline__ void gauss_z_pair(const float* __restrict__ w, const 
 }
 
 // r = c - 0.5 |W^T x - b|^2 for one point and one cluster whose transposed factor and b are staged in shared memory
-template <int DP>
+template <int E>
 __device__ __forceinline__ float gauss_r_pairs(const float* __restrict__ sW, const float* __restrict__ sbv,
-                                               const uint64_t (&x2)[DP / 2], float c)
+                                               const uint64_t (&x2)[E / 2], float c)
 {
     float q = 0.f;
 #pragma unroll 2
-    for (int j = 0; j < DP; j += 2) {
+    for (int j = 0; j < E; j += 2) {
         float z0, z1;
-        gauss_z_pair<DP>(sW + j * DP, sbv + j, x2, z0, z1);
+        gauss_z_pair<E>(sW + j * E, sbv + j, x2, z0, z1);
         q = fmaf(z0, z0, q);
         q = fmaf(z1, z1, q);
     }
@@ -198,12 +198,12 @@ constexpr size_t kLabelSmemCap = 220 * 1024;
 // Shape of the label kernel for blocks of P points: a thread per point and KB clusters staged between two barriers
 // (16 KB of factors, at least one cluster).  At N = 1e6, D = 7, K = 30 this takes 215 us; two points per thread took
 // 190, but in batches of small data sets 117 against 48, and reading the factors through the L1 cache 284.
-template <int DP, int P>
+template <int E, int P>
 struct LabelTile {
-    static constexpr int KB = DP * DP * 4 >= 16384 ? 1 : 16384 / (DP * DP * 4);
-    static constexpr int F4 = DP * DP / 4;
+    static constexpr int KB = E * E * 4 >= 16384 ? 1 : 16384 / (E * E * 4);
+    static constexpr int F4 = E * E / 4;
     // shared memory in bytes: kb factors and biases, then r [K][P]; kb: KB, or what the cap leaves beside a large K
-    static size_t bytes(int K, int kb) { return sizeof(float) * ((size_t)kb * (DP * DP + DP) + (size_t)K * P); }
+    static size_t bytes(int K, int kb) { return sizeof(float) * ((size_t)kb * (E * E + E) + (size_t)K * P); }
     static int staged(int K)
     {
         int kb = KB < K ? KB : K;
@@ -216,7 +216,10 @@ struct LabelTile {
 // the factors from shared memory (16 bytes for two packed multiply-adds and point) and, where the clusters overlap,
 // the draws.  Barriers come once per KB clusters and the points go straight to registers, so that several blocks
 // fit an SM: N = 1e5, D = 100, K = 12 2200 -> 1320 us; N = 1e6, D = 7, K = 30 236 -> 215 us.
-template <int DP, int P>
+// Features from D on are zero in the points and rows from D on give z = 0, so sums end exactly where they stand after
+// the first E >= D features and rows.  At Dp = 128 E is D rounded up to 16 (the same case at E = 112: 1023 us);
+// narrower widths have at most 31 padded features and use E = DP.
+template <int DP, int P, int E>
 __device__ __forceinline__ void gauss_labels_tile(const float* __restrict__ x, int64_t N,
                                                   const float* __restrict__ Wt, const float* __restrict__ bvec,
                                                   const float* __restrict__ cvec, int K, int final_,
@@ -224,19 +227,19 @@ __device__ __forceinline__ void gauss_labels_tile(const float* __restrict__ x, i
                                                   float* __restrict__ r_out, int64_t pt0, int kb,
                                                   unsigned char* smem)
 {
-    using L = LabelTile<DP, P>;
-    float* sW = reinterpret_cast<float*>(smem);           // kb * DP*DP
-    float* sbv = sW + (size_t)kb * DP * DP;               // kb * DP
-    float* sr = sbv + (size_t)kb * DP;                    // K*P
+    using L = LabelTile<E, P>;
+    float* sW = reinterpret_cast<float*>(smem);           // kb * E*E
+    float* sbv = sW + (size_t)kb * E * E;               // kb * E
+    float* sr = sbv + (size_t)kb * E;                    // K*P
 
     const int t = threadIdx.x;
     const int64_t pt = pt0 + t;
     const bool valid = pt < N;
-    uint64_t x2[DP / 2];
+    uint64_t x2[E / 2];
     {
         const ulonglong2* src = reinterpret_cast<const ulonglong2*>(x + min(pt, N - 1) * DP);
 #pragma unroll
-        for (int i4 = 0; i4 < DP / 4; ++i4) {
+        for (int i4 = 0; i4 < E / 4; ++i4) {
             const ulonglong2 v = __ldg(src + i4);
             x2[2 * i4] = v.x;
             x2[2 * i4 + 1] = v.y;
@@ -246,14 +249,14 @@ __device__ __forceinline__ void gauss_labels_tile(const float* __restrict__ x, i
         const int nk = min(kb, K - k0);
         __syncthreads();
         for (int e = t; e < nk * L::F4; e += P) {
-            const int kk = e / L::F4;
-            reinterpret_cast<float4*>(sW)[e] = reinterpret_cast<const float4*>(Wt + (size_t)3 * (k0 + kk) * DP * DP)[e % L::F4];
+            const int kk = e / L::F4, j = e % L::F4 / (E / 4), i4 = e % (E / 4);
+            reinterpret_cast<float4*>(sW)[e] = reinterpret_cast<const float4*>(Wt + (size_t)3 * (k0 + kk) * DP * DP)[j * (DP / 4) + i4];
         }
-        for (int e = t; e < nk * DP; e += P) sbv[e] = bvec[(size_t)3 * (k0 + e / DP) * DP + e % DP];
+        for (int e = t; e < nk * E; e += P) sbv[e] = bvec[(size_t)3 * (k0 + e / E) * DP + e % E];
         __syncthreads();
         for (int kk = 0; kk < nk; ++kk) {
             const int k = k0 + kk;
-            const float r = gauss_r_pairs<DP>(sW + (size_t)kk * DP * DP, sbv + kk * DP, x2, cvec[3 * k]);
+            const float r = gauss_r_pairs<E>(sW + (size_t)kk * E * E, sbv + kk * E, x2, cvec[3 * k]);
             sr[k * P + t] = r;
             if (r_out && valid) r_out[pt * K + k] = r;
         }
@@ -261,14 +264,14 @@ __device__ __forceinline__ void gauss_labels_tile(const float* __restrict__ x, i
     if (valid) labels[pt] = draw_from_r<P>(sr, t, K, final_, rng, pt);
 }
 
-template <int DP, int P>
+template <int DP, int P, int E>
 __global__ void __launch_bounds__(P) k_gauss_labels_simt(
     const float* __restrict__ x, int64_t N, const float* __restrict__ Wt, const float* __restrict__ bvec,
     const float* __restrict__ cvec, int K, int final_, RngArgs rng, int32_t* __restrict__ labels,
     float* __restrict__ r_out, int kb)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    gauss_labels_tile<DP, P>(x, N, Wt, bvec, cvec, K, final_, rng, labels, r_out, (int64_t)blockIdx.x * P, kb, smem);
+    gauss_labels_tile<DP, P, E>(x, N, Wt, bvec, cvec, K, final_, rng, labels, r_out, (int64_t)blockIdx.x * P, kb, smem);
 }
 
 // Batched form: one launch for many data sets of the same padded dimension.  Block b works on
@@ -281,7 +284,7 @@ __global__ void __launch_bounds__(P) k_gauss_labels_batched(const LabelJob* __re
     extern __shared__ __align__(16) unsigned char smem[];
     const int2 it = items[blockIdx.x];
     const LabelJob& j = jobs[it.x];
-    gauss_labels_tile<DP, P>(j.x, j.N, j.Wt, j.b, j.c, j.K, j.final_, j.rng, j.labels, nullptr, (int64_t)it.y * P,
+    gauss_labels_tile<DP, P, DP>(j.x, j.N, j.Wt, j.b, j.c, j.K, j.final_, j.rng, j.labels, nullptr, (int64_t)it.y * P,
                              kb, smem);
 }
 
@@ -395,17 +398,28 @@ __global__ void __launch_bounds__(256) k_mult_labels_simt(
     labels[pt] = draw_from_r<P>(sr, tid, K, final_, rng, pt);
 }
 
-template <int DP, int P>
-static dpmm_status launch_gauss_labels_t(dpmm_ctx* c, int K, int final_, RngArgs r, float* d_rout)
+template <int DP, int P, int E>
+static dpmm_status launch_gauss_labels_e(dpmm_ctx* c, int K, int final_, RngArgs r, float* d_rout)
 {
-    const int kb = LabelTile<DP, P>::staged(K);
-    const size_t sm = LabelTile<DP, P>::bytes(K, kb);
-    auto kern = k_gauss_labels_simt<DP, P>;
+    const int kb = LabelTile<E, P>::staged(K);
+    const size_t sm = LabelTile<E, P>::bytes(K, kb);
+    auto kern = k_gauss_labels_simt<DP, P, E>;
     DPMM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     kern<<<blocks_for(c->N, P), P, sm, c->stream>>>(c->d_x, c->N, c->d_Wt, c->d_b, c->d_c, K, final_, r,
                                                      c->d_labels, d_rout, kb);
     DPMM_LAUNCHED();
     return DPMM_OK;
+}
+
+template <int DP, int P>
+static dpmm_status launch_gauss_labels_t(dpmm_ctx* c, int K, int final_, RngArgs r, float* d_rout)
+{
+    if constexpr (DP == 128) {
+        if (c->D <= 80) return launch_gauss_labels_e<DP, P, 80>(c, K, final_, r, d_rout);
+        if (c->D <= 96) return launch_gauss_labels_e<DP, P, 96>(c, K, final_, r, d_rout);
+        if (c->D <= 112) return launch_gauss_labels_e<DP, P, 112>(c, K, final_, r, d_rout);
+    }
+    return launch_gauss_labels_e<DP, P, DP>(c, K, final_, r, d_rout);
 }
 
 template <int DP>
@@ -1464,8 +1478,9 @@ __global__ void __launch_bounds__(256, (DP <= 8 ? 4 : DP == 16 ? 3 : 2)) k_gauss
 // Draws: one block per tile of 128 points of a chunk; warps 0-3 evaluate the l factor, warps 4-7 the r factor, a thread
 // per point with x - s in registers.  The factors are transposed in shared memory, so that four outputs come
 // with one 16-byte read and two go through one packed multiply-add; each z_j stays one chain over the features, and
-// |z|^2 one chain over j.  Bound: those reads.
+// |z|^2 one chain over j.  E: D rounded up to 16, as in gauss_labels_tile.  Bound: those reads.
 constexpr int kWideLD = 132;   // shared row stride of 128 floats (16-byte rows)
+template <int E>
 __global__ void __launch_bounds__(256, 1) k_gauss_sub_draw_wide(
     const float* __restrict__ x, const int32_t* __restrict__ perm, const int32_t* __restrict__ chunk,
     const int32_t* __restrict__ nchunks, const float* __restrict__ Wt, const float* __restrict__ bvec,
@@ -1474,35 +1489,36 @@ __global__ void __launch_bounds__(256, 1) k_gauss_sub_draw_wide(
 {
     constexpr int DP = 128, TP = 128;
     extern __shared__ __align__(16) unsigned char smem[];
-    float* sW = reinterpret_cast<float*>(smem);       // [2][i][kWideLD]: W(i, j), j contiguous
-    float* sb = sW + 2 * DP * kWideLD;                // [2][DP] b - W^T s
-    float* ss = sb + 2 * DP;                          // [DP] s, the cluster's mean parameter
-    float* sq = ss + DP;                              // [2][TP]
+    constexpr int LD = E + 4;                         // 16-byte rows
+    float* sW = reinterpret_cast<float*>(smem);       // [2][i][LD]: W(i, j), j contiguous
+    float* sb = sW + 2 * E * LD;                      // [2][E] b - W^T s
+    float* ss = sb + 2 * E;                           // [E] s, the cluster's mean parameter
+    float* sq = ss + E;                               // [2][TP]
     const int ch = blockIdx.x, t0 = (int)blockIdx.y * TP;
     if (ch >= *nchunks) return;
     const int k = chunk[3 * ch], start = chunk[3 * ch + 1], len = chunk[3 * ch + 2];
     if (t0 >= len || (mask && !mask[k])) return;
     const int tid = threadIdx.x, side = tid >> 7, pp = tid & 127;
     const int64_t pt = perm[start + min(t0 + pp, len - 1)];
-    for (int e = tid; e < 2 * DP * DP / 4; e += 256) {
-        const int sd = e / (DP * DP / 4), j = e / (DP / 4) % DP, i4 = e % (DP / 4);
+    for (int e = tid; e < 2 * E * E / 4; e += 256) {
+        const int sd = e / (E * E / 4), j = e / (E / 4) % E, i4 = e % (E / 4);
         const float4 v = reinterpret_cast<const float4*>(Wt + (size_t)(3 * k + 1 + sd) * DP * DP)[j * (DP / 4) + i4];
-        float* dst = sW + (size_t)(sd * DP + 4 * i4) * kWideLD + j;
+        float* dst = sW + (size_t)(sd * E + 4 * i4) * LD + j;
         dst[0] = v.x;
-        dst[kWideLD] = v.y;
-        dst[2 * kWideLD] = v.z;
-        dst[3 * kWideLD] = v.w;
+        dst[LD] = v.y;
+        dst[2 * LD] = v.z;
+        dst[3 * LD] = v.w;
     }
-    if (tid < DP) ss[tid] = muv[(size_t)(3 * k) * DP + tid];
+    if (tid < E) ss[tid] = muv[(size_t)(3 * k) * DP + tid];
     __syncthreads();
-    {
+    if (pp < E) {
         float acc = 0.f;
-        for (int i = 0; i < DP; ++i) acc = fmaf(sW[(side * DP + i) * kWideLD + pp], ss[i], acc);
-        sb[side * DP + pp] = bvec[(size_t)(3 * k + 1 + side) * DP + pp] - acc;
+        for (int i = 0; i < E; ++i) acc = fmaf(sW[(side * E + i) * LD + pp], ss[i], acc);
+        sb[side * E + pp] = bvec[(size_t)(3 * k + 1 + side) * DP + pp] - acc;
     }
-    float xr[DP];
+    float xr[E];
 #pragma unroll
-    for (int i4 = 0; i4 < DP / 4; ++i4) {
+    for (int i4 = 0; i4 < E / 4; ++i4) {
         const float4 v = __ldg(reinterpret_cast<const float4*>(x + pt * DP) + i4);
         const float4 s4 = *reinterpret_cast<const float4*>(ss + 4 * i4);
         xr[4 * i4] = v.x - s4.x;
@@ -1511,16 +1527,16 @@ __global__ void __launch_bounds__(256, 1) k_gauss_sub_draw_wide(
         xr[4 * i4 + 3] = v.w - s4.w;
     }
     __syncthreads();
-    const float* Ws = sW + (size_t)side * DP * kWideLD;
+    const float* Ws = sW + (size_t)side * E * LD;
     float q = 0.f;
 #pragma unroll 1
-    for (int j0 = 0; j0 < DP; j0 += 16) {
+    for (int j0 = 0; j0 < E; j0 += 16) {
         uint64_t z[8];
 #pragma unroll
-        for (int m = 0; m < 8; ++m) z[m] = pack2(-sb[side * DP + j0 + 2 * m], -sb[side * DP + j0 + 2 * m + 1]);
+        for (int m = 0; m < 8; ++m) z[m] = pack2(-sb[side * E + j0 + 2 * m], -sb[side * E + j0 + 2 * m + 1]);
 #pragma unroll
-        for (int i = 0; i < DP; ++i) {
-            const ulonglong2* w = reinterpret_cast<const ulonglong2*>(Ws + i * kWideLD + j0);
+        for (int i = 0; i < E; ++i) {
+            const ulonglong2* w = reinterpret_cast<const ulonglong2*>(Ws + i * LD + j0);
             const uint64_t xi = pack2(xr[i], xr[i]);
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
@@ -1551,14 +1567,15 @@ __global__ void __launch_bounds__(256, 1) k_gauss_sub_draw_wide(
 // Statistics (the sub-labels are given): a block per chunk and sub-cluster; each of 136 threads owns an 8 x 8 block of
 // the upper triangle (the diagonal ones the sums too) and adds the side's points of every window of 32 points in FP32,
 // two columns per packed multiply-add, then the window into FP64 totals in registers.  Bound: the multiply-adds (32 a
-// point and thread).  With the draws, N = 1e5, D = 100, K = 12: 2515 -> 640 us (one matrix entry at a time through a
+// point and thread).  With the draws, N = 1e5, D = 100, K = 12: 2515 -> 542 us (one matrix entry at a time through a
 // pair table, 33 entries a thread, and the draws by one half of the threads before).
 __global__ void __launch_bounds__(160) k_gauss_stats_wide(
     const float* __restrict__ x, const int32_t* __restrict__ perm, const int32_t* __restrict__ chunk,
     const int32_t* __restrict__ nchunks, const float* __restrict__ muv, const int32_t* __restrict__ sub,
-    double* __restrict__ part, const uint8_t* __restrict__ mask)
+    double* __restrict__ part, const uint8_t* __restrict__ mask, int D)
 {
-    constexpr int DP = 128, T = tri(DP), SL = 1 + DP + T, NB = DP / 8, TP = 64;
+    constexpr int DP = 128, T = tri(DP), SL = 1 + DP + T, TP = 64;
+    const int NB = (D + 7) / 8;   // blocks a side that hold features; the rest of the record is zero
     __shared__ __align__(16) float sx[TP * kWideLD];
     __shared__ __align__(16) float ss[DP];
     __shared__ int32_t ssub[TP];
@@ -1639,6 +1656,10 @@ __global__ void __launch_bounds__(160) k_gauss_stats_wide(
     }
     double* po = part + ((size_t)ch * 2 + (slot - 1)) * SL;
     if (tid == 0) po[0] = (double)cnt;
+    for (int j = 8 * NB + tid; j < DP; j += 160) {
+        po[1 + j] = 0.0;
+        for (int i = 0; i <= j; ++i) po[1 + DP + tri_index(DP, i, j)] = 0.0;
+    }
     if (!own) return;
 #pragma unroll
     for (int a = 0; a < 8; ++a)
@@ -2043,18 +2064,28 @@ static dpmm_status launch_mult_sub_stats_t(dpmm_ctx* c, RngArgs r, float* d_rout
     return DPMM_OK;
 }
 
+template <int E>
+static dpmm_status launch_gauss_sub_draw_wide(dpmm_ctx* c, RngArgs r, float* d_rout, const uint8_t* d_mask)
+{
+    constexpr size_t sm = sizeof(float) * (2 * E * (E + 4) + 3 * E + 2 * 128);
+    DPMM_CUDA_TRY(cudaFuncSetAttribute(k_gauss_sub_draw_wide<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    const dim3 grid((unsigned)c->max_chunks, (unsigned)((c->chunk_len + 127) / 128));
+    k_gauss_sub_draw_wide<E><<<grid, 256, sm, c->stream>>>(c->d_x, c->d_perm, c->d_chunk, c->d_nchunks, c->d_Wt, c->d_b, c->d_c,
+                                                           c->d_lrw, c->d_mu, r, c->d_sub, d_rout, d_mask);
+    DPMM_LAUNCHED();
+    return DPMM_OK;
+}
+
 static dpmm_status launch_gauss_sub_stats_wide(dpmm_ctx* c, int draw, RngArgs r, float* d_rout, const uint8_t* d_mask)
 {
     if (draw) {
-        constexpr size_t sm = sizeof(float) * (2 * 128 * kWideLD + 3 * 128 + 2 * 128);
-        DPMM_CUDA_TRY(cudaFuncSetAttribute(k_gauss_sub_draw_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        const dim3 grid((unsigned)c->max_chunks, (unsigned)((c->chunk_len + 127) / 128));
-        k_gauss_sub_draw_wide<<<grid, 256, sm, c->stream>>>(c->d_x, c->d_perm, c->d_chunk, c->d_nchunks, c->d_Wt, c->d_b, c->d_c,
-                                                            c->d_lrw, c->d_mu, r, c->d_sub, d_rout, d_mask);
-        DPMM_LAUNCHED();
+        if (c->D <= 80) DPMM_TRY(launch_gauss_sub_draw_wide<80>(c, r, d_rout, d_mask));
+        else if (c->D <= 96) DPMM_TRY(launch_gauss_sub_draw_wide<96>(c, r, d_rout, d_mask));
+        else if (c->D <= 112) DPMM_TRY(launch_gauss_sub_draw_wide<112>(c, r, d_rout, d_mask));
+        else DPMM_TRY(launch_gauss_sub_draw_wide<128>(c, r, d_rout, d_mask));
     }
     k_gauss_stats_wide<<<dim3((unsigned)c->max_chunks, 2), 160, 0, c->stream>>>(c->d_x, c->d_perm, c->d_chunk, c->d_nchunks,
-                                                                               c->d_mu, c->d_sub, c->d_part, d_mask);
+                                                                               c->d_mu, c->d_sub, c->d_part, d_mask, c->D);
     DPMM_LAUNCHED();
     return DPMM_OK;
 }

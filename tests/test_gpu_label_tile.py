@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("D,K", [(3, 255), (3, 256), (3, 257), (8, 1), (8, 63), (8, 64), (8, 65), (8, 400), (8, 800),
                                  (13, 15), (13, 16), (13, 17), (13, 33), (13, 420), (32, 3), (32, 4), (32, 5),
-                                 (50, 1), (50, 2), (50, 300), (100, 3), (128, 40), (128, 300)])
+                                 (50, 1), (50, 2), (50, 300), (65, 7), (80, 3), (81, 9), (100, 3), (113, 2), (128, 40), (128, 300)])
 @pytest.mark.parametrize("N", [1, 300])
 def test_stages(D, K, N):
     rng = np.random.default_rng(D * 1000 + K)

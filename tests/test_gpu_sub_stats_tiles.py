@@ -12,7 +12,7 @@ from oracle import oracle as O
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("D", [2, 4, 7, 8, 13, 16, 32, 60, 65, 100, 128])
+@pytest.mark.parametrize("D", [2, 4, 7, 8, 13, 16, 32, 60, 65, 80, 81, 97, 112, 113, 128])
 @pytest.mark.parametrize("K,lo,hi", [(9, 1, 300), (4, 127, 129), (5, 31, 33), (1, 1, 1)])
 def test_tiles(D, K, lo, hi):
     rng = np.random.default_rng(100 * D + K)
