@@ -11,8 +11,8 @@
 // of the reference (cudaKernel.cu:374-424, 27-124) in a second kernel, one thread per point.
 //
 // CTA roles (608 threads, persistent over 256-point super-tiles): warp 0 streams the A tiles
-// (points, packed at upload) and the B tiles (2 clusters = 128 columns, hi + lo, 32 KB, stored
-// pre-swizzled) with cp.async.bulk; warp 1 allocates TMEM; warps 1-2 each issue the 12
+// (points, packed at upload) and the B tiles (2 clusters of 64 columns or 4 of 32, stored
+// pre-swizzled) with cp.async.bulk; warp 1 allocates TMEM; warps 1-2 each issue the
 // tcgen05.mma (M=128, N=128, K=16) of one 128-point half per N tile into 2 accumulator pairs;
 // warps 3-18 drain the accumulators into r.
 // Every mbarrier wait is bounded: on timeout the CTA records an error code, stops issuing work,
@@ -20,8 +20,7 @@
 //
 // Operand layout: K-major, 128-byte swizzle (8-row x 128-byte atoms, 16-byte chunk c of row r
 // stored at chunk c ^ (r % 8)), descriptor SBO = 1024 B; a K-step of 16 elements advances the
-// descriptor start address by 32 bytes.  The padded dimension must be 32 or 64 (zero-filled
-// to 64).
+// descriptor start address by 32 bytes.  The padded dimension must be 32 or 64.
 #include <algorithm>
 
 #include "dpmm_tc.cuh"
@@ -168,9 +167,9 @@ __global__ void k_pack_b32(const float* __restrict__ Wt, int K, int NT, uint8_t*
 // 256 points (two 128-point tiles sharing every B tile, which halves the B traffic and the MMA
 // issue overhead per point).
 //
-//   warp 0      producer: A super-tile (64 KB, with an L2 prefetch of the next one), B tiles
-//               (32 KB) into a B ring, bias records into a bias ring
-//   warps 1-2   MMA issuers: per N tile 12 tcgen05.mma each (one per half) into pair g % 2
+//   warp 0      producer: the biases (once), A super-tile (with an L2 prefetch of the next one),
+//               B tiles into a B ring
+//   warps 1-2   MMA issuers: per N tile 12 tcgen05.mma each (6 at Dp = 32; one half a warp) into pair g % 2
 //   warps 3-18  drain: TMEM accumulator -> r = c - |z|^2 / 2 for one (lane quarter, cluster,
 //               half) per warp, written cluster-major to rbuf[k][point] (32 points per store),
 //               with a running max / sum of exp (or the first maximum, final mode) per point and
