@@ -181,12 +181,14 @@ struct AliasAcc {
 // reference's float->double promotions replaced by float maths.  Of the two exponentials one is exp(0) = 1
 // and the other e <= 1, s = 1 + e their sum.  Only the smaller category, y = 2 e / s < 1, can go to the other,
 // and only when that one has an excess (2 / s > 1, that is s < 2); a larger one drawn keeps itself.  The
-// column of the first uniform (alias_column for n = 2) is 2 from the first float above 1 / 1.999999 on.
+// column of the first uniform (alias_column for n = 2) is 2 from the first float above 1 / 1.999999 on.  Where
+// the larger value is +inf the softmax is NaN, every comparison of the construction is false and the
+// column is kept; two values of -inf or a NaN give a NaN e with the same outcome.
 __device__ __forceinline__ int draw_sub_label(float rl, float rr, float u1, float u2)
 {
     const int col = u1 >= 0.50000029802322388f ? 2 : 1;
     const bool l_larger = rl >= rr;
-    if ((col == 1) == l_larger) return col;
+    if ((col == 1) == l_larger || fmaxf(rl, rr) == INFINITY) return col;
     const float e = __expf(-fabsf(rl - rr)), s = 1.0f + e;
     const float y = (e / s) * 2.0f;
     return s < 2.0f && y < 1.0f && y < u2 ? 3 - col : col;
