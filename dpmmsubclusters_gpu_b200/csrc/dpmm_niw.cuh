@@ -99,26 +99,30 @@ struct BlockChol {
 // Correctly rounded quotients by one divisor b: with y = RN(1 / b), a quotient q within an ulp of a / b and the
 // exact remainder a - b q, RN(q + (a - b q) y) is RN(a / b) (P. Markstein, "Computation of elementary functions
 // on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990, theorem on the final step of a
-// division); the first correction brings a y (two roundings) within the ulp.  Equal bit for bit to a / b for
-// quotients in the normal range, but without a branch, so that several quotients by one b run side by side
-// (6 dependent operations each after the reciprocal), where the compiler keeps two divisions one after the
-// other (a panel of 8 columns: 400 -> 190 clocks a column).  Both sides are scaled by the power of two that
-// brings b near 1: no product leaves the range for a very small or large b.
+// division); the first correction brings a y (two roundings) within the ulp.  No branch, so that several
+// quotients by one b run side by side (6 dependent operations each after the reciprocal), where the compiler
+// keeps two divisions one after the other (a panel of 8 columns: 400 -> 190 clocks a column).  Both sides are
+// scaled by the power of two that brings b to 1/4 .. 1/2: no product leaves the range where the quotient does not.
+// Equal bit for bit to a / b for quotients of 2^-960 and above in magnitude (below, the remainder is not exact
+// and the last two places may differ) and for zero, infinite and NaN operands and results: there the
+// corrections would make NaN of an infinity, and a y already is the quotient.
 struct Divisor {
     double b, y, scale;
     __device__ __forceinline__ explicit Divisor(double d)
     {
         const int e = (__double2hiint(d) >> 20) & 0x7ff;
-        scale = __hiloint2double((2046 - min(max(e, 2), 2045)) << 20, 0);
+        scale = __hiloint2double((2044 - min(e, 2043)) << 20, 0);
         b = d * scale;
         y = 1.0 / b;
     }
     __device__ __forceinline__ double operator()(double a) const
     {
         a *= scale;
-        double q = a * y;
-        q = fma(fma(-b, q, a), y, q);
-        return fma(fma(-b, q, a), y, q);
+        const double q0 = a * y;
+        const bool normal = (unsigned)(__double2hiint(q0) & 0x7ff00000) - 0x00100000u < 0x7fe00000u;
+        const double q1 = fma(fma(-b, q0, a), y, q0);
+        const double q2 = fma(fma(-b, q1, a), y, q1);
+        return normal ? q2 : q0;
     }
 };
 
