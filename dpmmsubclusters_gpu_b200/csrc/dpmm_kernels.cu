@@ -2055,7 +2055,8 @@ static dpmm_status launch_mult_sub_stats_t(dpmm_ctx* c, RngArgs r, float* d_rout
     const int R = mult_stage_rows(c->Dp);
     // the group sums reuse the stages: 8 KB at most
     const size_t sm = sizeof(float) * ((size_t)2 * c->Dp + std::max<size_t>((size_t)2 * R * c->Dp, 2048));
-    if (sm > 48 * 1024)
+    constexpr size_t arrays = sizeof(float) * 6 * kMultRows;   // the kernel's static ones count against the 48 KB too
+    if (sm + arrays > 48 * 1024)
         DPMM_CUDA_TRY(cudaFuncSetAttribute(k_mult_sub_stats<NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     k_mult_sub_stats<NG><<<c->max_chunks, 256, sm, c->stream>>>(c->d_x, c->Dp, c->d_perm, c->d_chunk, c->d_nchunks, c->d_mu,
                                                                c->d_lrw, draw, r, c->d_sub, d_rout, c->d_part, 1 + c->Dp,
