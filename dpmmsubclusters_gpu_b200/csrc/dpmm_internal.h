@@ -66,6 +66,23 @@ dpmm_status cuda_status(cudaError_t e, const char* what);
         if (_e != cudaSuccess) return ::dpmm::cuda_status(_e, #expr);    \
     } while (0)
 
+// A launch of more than 48 KB of shared memory, static arrays included, needs its kernel's limit raised first.  The
+// limit belongs to the function on the device, so contexts on other threads share it: it is always raised to
+// `cap`, the most that the kernel can ever ask for, and no thread takes it back between another's call and
+// launch.  (It does not touch residency: that follows the bytes of the launch.)  Set on every launch that needs it
+// rather than once, since cudaDeviceReset clears it.  No kernel here has 24 KB of static arrays.
+template <typename Kern>
+inline dpmm_status allow_smem(Kern k, size_t bytes, size_t cap)
+{
+    if (bytes > 24 * 1024) DPMM_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+    return DPMM_OK;
+}
+template <typename Kern>
+inline dpmm_status allow_smem(Kern k, size_t bytes)   // a kernel whose launches all ask for the same
+{
+    return allow_smem(k, bytes, bytes);
+}
+
 // process-wide diagnostics: kernels launched, bytes copied host->device / device->host
 extern std::atomic<uint64_t> g_launches, g_h2d_bytes, g_d2h_bytes;
 

@@ -302,7 +302,7 @@ static dpmm_status launch_labels_batched_t(const LabelJob* d_jobs, const int2* d
     const int kb = LabelTile<DP, P>::staged(kmax);
     const size_t sm = LabelTile<DP, P>::bytes(kmax, kb);
     auto kern = k_gauss_labels_batched<DP, P>;
-    DPMM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    DPMM_TRY(allow_smem(kern, sm, kLabelSmemCap));
     kern<<<nitems, P, sm, st>>>(d_jobs, d_items, kb);
     DPMM_LAUNCHED();
     return DPMM_OK;
@@ -404,7 +404,7 @@ static dpmm_status launch_gauss_labels_e(dpmm_ctx* c, int K, int final_, RngArgs
     const int kb = LabelTile<E, P>::staged(K);
     const size_t sm = LabelTile<E, P>::bytes(K, kb);
     auto kern = k_gauss_labels_simt<DP, P, E>;
-    DPMM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    DPMM_TRY(allow_smem(kern, sm, kLabelSmemCap));
     kern<<<blocks_for(c->N, P), P, sm, c->stream>>>(c->d_x, c->N, c->d_Wt, c->d_b, c->d_c, K, final_, r,
                                                      c->d_labels, d_rout, kb);
     DPMM_LAUNCHED();
@@ -447,8 +447,8 @@ dpmm_status launch_cluster_labels(dpmm_ctx* c, int K, int final_, const float* d
     }
     constexpr int P = 64;
     size_t sm = sizeof(float) * (P * 33 + 64 * 33 + (size_t)K * P);
-    if (sm > 220 * 1024) return fail(DPMM_ERR_INVALID_ARG, "too many clusters for the multinomial label kernel");
-    DPMM_CUDA_TRY(cudaFuncSetAttribute(k_mult_labels_simt<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    if (sm > kLabelSmemCap) return fail(DPMM_ERR_INVALID_ARG, "too many clusters for the multinomial label kernel");
+    DPMM_TRY(allow_smem(k_mult_labels_simt<P>, sm, kLabelSmemCap));
     k_mult_labels_simt<P><<<blocks_for(c->N, P), 256, sm, c->stream>>>(c->d_x, c->N, c->Dp, c->d_mu, K, final_, r,
                                                                        c->d_labels, d_rout);
     DPMM_LAUNCHED();
@@ -854,6 +854,7 @@ __global__ void __launch_bounds__(kPrTh) k_prune_draw(const float* __restrict__ 
     }
 }
 
+static size_t prune_scan_smem(int DP, int K) { return sizeof(float) * ((size_t)kChunkMax + (size_t)K * (DP + 3)); }
 static size_t prune_draw_smem(int DP, int K) { return sizeof(float) * ((size_t)DP * DP + DP + (size_t)K * kPrTh); }
 
 template <int DP>
@@ -872,8 +873,8 @@ static dpmm_status launch_pruned_dp(dpmm_ctx* c, int K, int final_, const float*
         KernelTimer kt(c, PH_PRUNE_SCAN);
         DPMM_TRY(launch_prune_scan_tc(c, K, d_err));
     } else {
-        const size_t ssm = sizeof(float) * ((size_t)kChunkMax + (size_t)K * (DP + 3));
-        DPMM_CUDA_TRY(cudaFuncSetAttribute(k_prune_scan<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm));
+        const size_t ssm = prune_scan_smem(DP, K);
+        DPMM_TRY(allow_smem(k_prune_scan<DP>, ssm, prune_scan_smem(DP, kMaxKForPrune)));
         KernelTimer kt(c, PH_PRUNE_SCAN);
         k_prune_scan<DP><<<c->max_chunks, kPrTh, ssm, c->stream>>>(
             c->d_x, c->d_perm, c->d_chunk, c->d_nchunks, c->d_Wt, c->d_b, c->d_c, c->d_mu, c->d_prune_lam,
@@ -910,7 +911,7 @@ static dpmm_status launch_pruned_dp(dpmm_ctx* c, int K, int final_, const float*
     }
     const RngArgs r = rng_args(c, d_u);
     const size_t sm = prune_draw_smem(DP, K);
-    DPMM_CUDA_TRY(cudaFuncSetAttribute(k_prune_draw<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    DPMM_TRY(allow_smem(k_prune_draw<DP>, sm, kLabelSmemCap));
     {
         KernelTimer kt(c, PH_PRUNE_DRAW);
         k_prune_settle<<<c->max_chunks, 256, 0, c->stream>>>(c->d_perm, c->d_chunk, c->d_nchunks, c->d_prune_cand,
@@ -940,7 +941,7 @@ dpmm_status launch_cluster_labels_pruned(dpmm_ctx* c, int K, int final_, const f
     // below kMinKForPruneTc clusters the tensor-core dense phase costs less than the scan alone
     const bool tc_dense = c->ll_mode != DPMM_LL_FP32 && tc_supported(c, K);
     if (tc_dense && K < kMinKForPruneTc) return DPMM_OK;
-    if (prune_draw_smem(c->Dp, K) > 220 * 1024) return DPMM_OK;
+    if (prune_draw_smem(c->Dp, K) > kLabelSmemCap) return DPMM_OK;
     if (c->prune_wait > 0) {
         --c->prune_wait;
         return DPMM_OK;
@@ -1134,7 +1135,7 @@ dpmm_status build_permutation(dpmm_ctx* c, int K)
                                          c->max_chunks, c->chunk_len);
     DPMM_LAUNCHED();
     size_t sm = sizeof(int32_t) * 9 * (K + 1);
-    if (sm > 48 * 1024) DPMM_CUDA_TRY(cudaFuncSetAttribute(k_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    DPMM_TRY(allow_smem(k_scatter, sm, tc::kTcSmemCap));
     k_scatter<<<nblk, 256, sm, c->stream>>>(c->d_labels, c->N, K, c->d_blk_hist, c->d_seg, c->d_perm);
     DPMM_LAUNCHED();
     c->perm_K = K;
@@ -2048,6 +2049,7 @@ static int mult_stage_rows(int Dp)
     const int r = std::max(8, std::min(kMultRows, 8192 / Dp / 8 * 8));
     return 2 * r * Dp * 4 <= 160 * 1024 ? r : 4;
 }
+constexpr size_t kMultSmemCap = 180 * 1024;   // two stages of 80 KB and both rows of log theta, 20 KB at Dp = 2560 (32 KB beside two of 64 KB at 4096)
 
 template <int NG>
 static dpmm_status launch_mult_sub_stats_t(dpmm_ctx* c, RngArgs r, float* d_rout, int draw, const uint8_t* d_mask)
@@ -2055,9 +2057,7 @@ static dpmm_status launch_mult_sub_stats_t(dpmm_ctx* c, RngArgs r, float* d_rout
     const int R = mult_stage_rows(c->Dp);
     // the group sums reuse the stages: 8 KB at most
     const size_t sm = sizeof(float) * ((size_t)2 * c->Dp + std::max<size_t>((size_t)2 * R * c->Dp, 2048));
-    constexpr size_t arrays = sizeof(float) * 6 * kMultRows;   // the kernel's static ones count against the 48 KB too
-    if (sm + arrays > 48 * 1024)
-        DPMM_CUDA_TRY(cudaFuncSetAttribute(k_mult_sub_stats<NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    DPMM_TRY(allow_smem(k_mult_sub_stats<NG>, sm, kMultSmemCap));
     k_mult_sub_stats<NG><<<c->max_chunks, 256, sm, c->stream>>>(c->d_x, c->Dp, c->d_perm, c->d_chunk, c->d_nchunks, c->d_mu,
                                                                c->d_lrw, draw, r, c->d_sub, d_rout, c->d_part, 1 + c->Dp,
                                                                d_mask, R);
@@ -2069,7 +2069,7 @@ template <int E>
 static dpmm_status launch_gauss_sub_draw_wide(dpmm_ctx* c, RngArgs r, float* d_rout, const uint8_t* d_mask)
 {
     constexpr size_t sm = sizeof(float) * (2 * E * (E + 4) + 3 * E + 2 * 128);
-    DPMM_CUDA_TRY(cudaFuncSetAttribute(k_gauss_sub_draw_wide<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    DPMM_TRY(allow_smem(k_gauss_sub_draw_wide<E>, sm));
     const dim3 grid((unsigned)c->max_chunks, (unsigned)((c->chunk_len + 127) / 128));
     k_gauss_sub_draw_wide<E><<<grid, 256, sm, c->stream>>>(c->d_x, c->d_perm, c->d_chunk, c->d_nchunks, c->d_Wt, c->d_b, c->d_c,
                                                            c->d_lrw, c->d_mu, r, c->d_sub, d_rout, d_mask);
@@ -2099,7 +2099,7 @@ static dpmm_status launch_gauss_sub_stats_t(dpmm_ctx* c, int draw, RngArgs r, fl
         if (!draw) {
             const size_t sm = SlotStatsShape<DP>::bytes;
             auto kern = k_gauss_slot_stats<DP>;
-            DPMM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+            DPMM_TRY(allow_smem(kern, sm));
             KernelTimer kt(d_mask ? nullptr : c, PH_SLOT_STATS);   // full launches only (masked: a few clusters)
             kern<<<c->max_chunks, 256, sm, c->stream>>>(c->d_x, c->d_perm, c->d_chunk, c->d_nchunks, c->d_mu,
                                                         c->d_sub, c->d_part, d_mask);
@@ -2109,7 +2109,7 @@ static dpmm_status launch_gauss_sub_stats_t(dpmm_ctx* c, int draw, RngArgs r, fl
     }
     const size_t sm = SubStatsShape<DP>::bytes;
     auto kern = k_gauss_sub_stats<DP>;
-    DPMM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    DPMM_TRY(allow_smem(kern, sm));
     kern<<<c->max_chunks, 256, sm, c->stream>>>(c->d_x, c->d_perm, c->d_chunk, c->d_nchunks, c->d_Wt, c->d_b, c->d_c,
                                                 c->d_lrw, c->d_mu, draw, r, c->d_sub, d_rout, c->d_part, d_mask);
     DPMM_LAUNCHED();
@@ -2279,9 +2279,7 @@ dpmm_status launch_stats_finalize(dpmm_ctx* c, int K, const uint8_t* d_mask)
 {
     const int gauss = c->prior == DPMM_PRIOR_GAUSSIAN;
     const int SL = gauss ? 1 + c->Dp + tri(c->Dp) : 1 + c->Dp;
-    size_t sm = sizeof(double) * (2 + 3 * (size_t)c->D);
-    if (sm > 48 * 1024)
-        DPMM_CUDA_TRY(cudaFuncSetAttribute(k_stats_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    const size_t sm = gauss ? sizeof(double) * (2 + 3 * (size_t)c->D) : 0;   // at most 3 KB; the multinomial form uses none
     // a block's worth of values per share where K leaves room on the device
     const int values = gauss ? tri(c->Dp) : 1 + c->D;
     const dim3 grid((unsigned)K, (unsigned)std::max(1, std::min((values + 255) / 256, gauss ? 8 : 16)));

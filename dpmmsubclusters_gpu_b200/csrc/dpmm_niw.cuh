@@ -423,14 +423,6 @@ __device__ double merge_log_hr_block(const double* __restrict__ stats, int stat_
     default: { constexpr int DP = 128; body; } break;             \
     }
 
-// opt a kernel in to more than 48 KB of dynamic shared memory when it needs it
-template <typename Kern>
-static inline dpmm_status allow_smem(Kern k, size_t bytes)
-{
-    if (bytes > 48 * 1024) DPMM_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    return DPMM_OK;
-}
-
 // split log Hastings ratio of cluster k (local_clusters_actions.cpp:222-233) from the slot counts
 // and the log marginal likelihoods of slots 3k, 3k+1, 3k+2; NaN when a sub-cluster is empty
 static __device__ double split_log_hr_slot(const double* __restrict__ stats, int stat_len,

@@ -405,7 +405,7 @@ static dpmm_status launch_sub_labels_tc_t(dpmm_ctx* c, RngArgs r, float* d_rout,
 {
     auto kern = tc::k_sub_labels_tc<DP>;
     static_assert(tc::SubSmem<DP>::total <= tc::kTcSmemCap, "shared memory");
-    DPMM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::SubSmem<DP>::total));
+    DPMM_TRY(allow_smem(kern, tc::SubSmem<DP>::total));
     kern<<<std::min(c->num_sms, c->max_chunks), tc::RW_THREADS, tc::SubSmem<DP>::total, c->stream>>>(
         c->d_x, c->d_perm, c->d_chunk, c->d_nchunks, DP == 32 ? c->d_Bsub32 : c->d_Bsub, c->d_b, c->d_c, c->d_lrw, r,
         c->d_sub, d_rout, err, c->stall_tc_mma);

@@ -1197,8 +1197,7 @@ size_t train_smem() { return sizeof(float) * kTrainSmemFloats; }
 
 dpmm_status enable_train_smem()
 {
-    DPMM_CUDA_TRY(cudaFuncSetAttribute(k_mlp_grad_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)train_smem()));
-    return DPMM_OK;
+    return allow_smem(k_mlp_grad_tile, train_smem());
 }
 
 }  // namespace

@@ -510,8 +510,7 @@ template <int NW, bool STAGED>
 static dpmm_status launch_draw_labels_t(dpmm_ctx* c, int K, int final_, const RngArgs& r)
 {
     const size_t sm = STAGED && !final_ ? sizeof(float) * 256 * (size_t)K : 0;
-    if (sm > 48 * 1024)
-        DPMM_CUDA_TRY(cudaFuncSetAttribute(k_draw_labels<NW, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    DPMM_TRY(allow_smem(k_draw_labels<NW, STAGED>, sm, sizeof(float) * 256 * 32 * NW));   // K <= 32 NW
     k_draw_labels<NW, STAGED><<<(unsigned)((c->N + 255) / 256), 256, sm, c->stream>>>(c->d_rbuf, c->d_rpart, c->N, K, final_, r,
                                                                                     c->d_labels);
     DPMM_LAUNCHED();
@@ -2162,7 +2161,7 @@ static dpmm_status launch_labels_tc_t(dpmm_ctx* c, int K, int final_, float* d_r
     for (int k0 = 0; k0 < K; k0 += tc::LABEL_PASS) {
         const int k1 = std::min(K, k0 + tc::LABEL_PASS), bstages = tc_stages<DP>(k1 - k0);
         const tc::SmemLayout L = tc::smem_layout<DP>(bstages, (k1 - k0 + O::CPT - 1) / O::CPT);
-        DPMM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total));
+        DPMM_TRY(allow_smem(kern, L.total, tc::kTcSmemCap));
         kern<<<grid, tc::THREADS, L.total, c->stream>>>(c->d_Atc, c->N, (int)ntiles, B + (size_t)(k0 / O::CPT) * O::B,
                                                         tc_bias_base(c) + (size_t)(k0 / O::CPT) * tc::BIAS_REC, k0, k1,
                                                         bstages, final_, c->d_rbuf, c->d_rpart, d_rout, K, err,
@@ -2199,7 +2198,7 @@ static dpmm_status launch_prune_scan_tc_t(dpmm_ctx* c, int K, int32_t* err)
 {
     // single pass while [W_h | every other cluster's v] fits two B tiles, else the two-pass form
     auto kern = K - 1 <= tc::kScan1MaxCand ? tc::k_prune_scan1_tc<DP> : tc::k_prune_scan_tc<DP>;
-    DPMM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::ScanSmem::total));
+    DPMM_TRY(allow_smem(kern, tc::ScanSmem::total));
     kern<<<c->max_chunks, 256, tc::ScanSmem::total, c->stream>>>(
         c->d_x, c->d_perm, c->d_chunk, c->d_nchunks, c->d_Btc, c->d_b, c->d_c, c->d_mu, c->d_prune_lam, c->d_prune_M,
         c->d_prune_V, c->d_prune_beta, K, c->prune_margin, c->d_prune_rh, c->d_prune_cand, c->d_prune_cnt, err,
@@ -2226,7 +2225,7 @@ static dpmm_status launch_slot_stats_tc_t(dpmm_ctx* c, const uint8_t* d_mask, in
 {
     auto kern = tc::k_slot_stats_tc<DP>;
     constexpr size_t sm = tc::StatSmem<DP>::total;
-    DPMM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    DPMM_TRY(allow_smem(kern, sm));
     kern<<<c->max_chunks, 256, sm, c->stream>>>(c->d_x, c->d_perm, c->d_chunk, c->d_nchunks, c->d_mu, c->d_sub,
                                                 c->d_part, d_mask, err, c->stall_tc_mma);
     DPMM_LAUNCHED();
@@ -2262,7 +2261,7 @@ static dpmm_status launch_sub_stats_tc_t(dpmm_ctx* c, RngArgs r, float* d_rout, 
 {
     auto kern = tc::k_sub_stats_tc<DP>;
     constexpr size_t sm = tc::SubStatSmem<DP>::total;
-    DPMM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    DPMM_TRY(allow_smem(kern, sm));
     kern<<<c->max_chunks, tc::SS_THREADS, sm, c->stream>>>(c->d_x, c->d_perm, c->d_chunk, c->d_nchunks, c->d_Bsub,
                                                             c->d_b, c->d_c, c->d_lrw, c->d_mu, r, c->d_sub, d_rout,
                                                             c->d_part, err, c->stall_tc_mma);
@@ -2623,7 +2622,7 @@ dpmm_status launch_mult_labels_tc(dpmm_ctx* c, int K, int final_, const float* d
     if (c->mult_tc_K != K) DPMM_TRY(pack_mult_tc_params(c, K));
     const int Kp = mt_kp(K), stages = mt_stages(Kp);
     const size_t sm = 1024 + (size_t)stages * tc::mt_stage_bytes(Kp) + (2 * tc::MT_MAX_STAGES + 4) * 8 + 16;
-    DPMM_CUDA_TRY(cudaFuncSetAttribute(tc::k_mult_labels_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    DPMM_TRY(allow_smem(tc::k_mult_labels_tc, sm, tc::kTcSmemCap));
     int32_t* err = c->d_aux + 7;
     DPMM_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int32_t), c->stream));
     const int64_t ntiles = (c->N + tc::BM - 1) / tc::BM;
