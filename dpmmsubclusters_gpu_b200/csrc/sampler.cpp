@@ -1547,12 +1547,21 @@ static dpmm_status batch_labels(dpmm_batch& b, dpmm_batch::Group& g, const std::
     for (size_t j = 0; j < mem.size(); ++j) kmax = std::max(kmax, g.h_jobs[j].K);
     if (g.P == 0 || kmax >= 2 * g.tuned_K) {
         // first iteration, and whenever the largest job has doubled its clusters since (what one cluster
-        // favours, the staging of many punishes): time every block size on the live jobs (each run draws the
-        // same labels: a point's log-likelihoods and uniforms do not depend on the block size), keep the fastest
+        // favours, the staging of many punishes): time every block size on the live jobs, keep the fastest.
+        // Each run draws the same labels: a point's log-likelihoods and uniforms do not depend on the block size.
+        // A job that draws from per-point states, which a launch moves on, is timed with counter-based
+        // uniforms instead, and the phase's own launch follows.
+        std::vector<LabelJob> timed(g.h_jobs, g.h_jobs + mem.size());
+        bool stateful = false;
+        for (LabelJob& j : timed)
+            if (j.rng.kind == DPMM_RNG_CURAND_XORWOW) {
+                j.rng.kind = DPMM_RNG_PHILOX;
+                stateful = true;
+            }
         cudaEvent_t e0, e1;
         DPMM_CUDA_TRY(cudaEventCreate(&e0));
         DPMM_CUDA_TRY(cudaEventCreate(&e1));
-        DPMM_CUDA_TRY(cudaMemcpyAsync(g.d_jobs, g.h_jobs, jb, cudaMemcpyHostToDevice, g.st));
+        DPMM_CUDA_TRY(cudaMemcpyAsync(g.d_jobs, timed.data(), jb, cudaMemcpyHostToDevice, g.st));
         int best = 0;
         for (int q = 0; q < 3; ++q) {
             DPMM_TRY(batch_items(b, g, mem, kBatchP[q]));
@@ -1573,6 +1582,11 @@ static dpmm_status batch_labels(dpmm_batch& b, dpmm_batch::Group& g, const std::
             g.graph = nullptr;
         }
         DPMM_TRY(batch_items(b, g, mem, g.P));
+        if (stateful) {
+            DPMM_CUDA_TRY(cudaMemcpyAsync(g.d_jobs, g.h_jobs, jb, cudaMemcpyHostToDevice, g.st));
+            DPMM_TRY(launch_labels_batched(g.Dp, g.P, g.d_jobs, g.d_items, g.nitems, g.kcap, g.st));
+            ++b.batched_launches;
+        }
         return DPMM_OK;
     }
     if (!g.graph || g.graph_members != mem) {
