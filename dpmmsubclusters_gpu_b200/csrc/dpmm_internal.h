@@ -340,7 +340,7 @@ struct LabelJob {
 // label phase of several Gaussian data sets of padded dimension Dp in one launch: nitems blocks of
 // P points, item (job, block); kmax: the largest K of the jobs
 dpmm_status launch_labels_batched(int Dp, int P, const LabelJob* d_jobs, const int2* d_items, int nitems, int kmax,
-                                  cudaStream_t st);
+                                  int num_sms, cudaStream_t st);
 size_t gauss_label_smem_bytes(int DP, int P, int K);
 // a context's label phase as a batch job (dpmm_capi.cu)
 dpmm_status make_label_job(dpmm_ctx* c, int K, int final_, LabelJob* job);

@@ -173,7 +173,8 @@ __device__ __forceinline__ float gauss_r_pairs(const float* __restrict__ sW, con
                                                const uint64_t (&x2)[E / 2], float c)
 {
     float q = 0.f;
-#pragma unroll 2
+    constexpr int U = E == 64 ? 1 : 2;   // E = 64: 4320 us unrolled twice, 4120 once (N = 1.2e5, K = 120; the scan 138 and 67)
+#pragma unroll U
     for (int j = 0; j < E; j += 2) {
         float z0, z1;
         gauss_z_pair<E>(sW + j * E, sbv + j, x2, z0, z1);
@@ -183,14 +184,41 @@ __device__ __forceinline__ float gauss_r_pairs(const float* __restrict__ sW, con
     return c - 0.5f * q;
 }
 
+// The same with x as single floats.  DP = 32: the same chains as single multiply-adds, since the packed form made
+// k_prune_scan<32>, a block of few points per chunk, wait longer for its factors (N = 2e4, K = 3: 52 against 39 us).
 template <int DP>
 __device__ __forceinline__ float gauss_r_point(const float* __restrict__ sW, const float* __restrict__ sbv,
                                                const float (&xr)[DP], float c)
 {
-    uint64_t x2[DP / 2];
+    if constexpr (DP == 32) {
+        float q = 0.f;
+#pragma unroll 2
+        for (int j = 0; j < DP; j += 2) {
+            const float4* w0 = reinterpret_cast<const float4*>(sW + j * DP);
+            const float4* w1 = reinterpret_cast<const float4*>(sW + (j + 1) * DP);
+            float e0 = -sbv[j], e1 = -sbv[j + 1], o0 = 0.f, o1 = 0.f;
 #pragma unroll
-    for (int i = 0; i < DP / 2; ++i) x2[i] = pack2(xr[2 * i], xr[2 * i + 1]);
-    return gauss_r_pairs<DP>(sW, sbv, x2, c);
+            for (int i4 = 0; i4 < DP / 4; ++i4) {
+                const float4 a = w0[i4], b = w1[i4];
+                e0 = fmaf(a.x, xr[4 * i4], e0);
+                e1 = fmaf(b.x, xr[4 * i4], e1);
+                o0 = fmaf(a.y, xr[4 * i4 + 1], o0);
+                o1 = fmaf(b.y, xr[4 * i4 + 1], o1);
+                e0 = fmaf(a.z, xr[4 * i4 + 2], e0);
+                e1 = fmaf(b.z, xr[4 * i4 + 2], e1);
+                o0 = fmaf(a.w, xr[4 * i4 + 3], o0);
+                o1 = fmaf(b.w, xr[4 * i4 + 3], o1);
+            }
+            q = fmaf(e0 + o0, e0 + o0, q);
+            q = fmaf(e1 + o1, e1 + o1, q);
+        }
+        return c - 0.5f * q;
+    } else {
+        uint64_t x2[DP / 2];
+#pragma unroll
+        for (int i = 0; i < DP / 2; ++i) x2[i] = pack2(xr[2 * i], xr[2 * i + 1]);
+        return gauss_r_pairs<DP>(sW, sbv, x2, c);
+    }
 }
 
 constexpr size_t kLabelSmemCap = 220 * 1024;
@@ -198,16 +226,22 @@ constexpr size_t kLabelSmemCap = 220 * 1024;
 // Shape of the label kernel for blocks of P points: a thread per point and KB clusters staged between two barriers
 // (16 KB of factors, at least one cluster).  At N = 1e6, D = 7, K = 30 this takes 215 us; two points per thread took
 // 190, but in batches of small data sets 117 against 48, and reading the factors through the L1 cache 284.
+// Where r [K][P] takes most of an SM's 228 KB, staging less keeps more blocks resident: as many as the launch has
+// for an SM, if one staged cluster allows it, and at most 8 (a KB per block is the system's).  N = 6e5, K = 120:
+// 2282 -> 1728 us at D = 8, 2540 -> 2030 at D = 16; with few blocks an SM nothing is gained (N = 2e4: 57 against 59).
 template <int E, int P>
 struct LabelTile {
     static constexpr int KB = E * E * 4 >= 16384 ? 1 : 16384 / (E * E * 4);
     static constexpr int F4 = E * E / 4;
     // shared memory in bytes: kb factors and biases, then r [K][P]; kb: KB, or what the cap leaves beside a large K
     static size_t bytes(int K, int kb) { return sizeof(float) * ((size_t)kb * (E * E + E) + (size_t)K * P); }
-    static int staged(int K)
+    static int staged(int K, int64_t blocks, int num_sms)
     {
+        constexpr size_t sm = 228 * 1024, own = 1024;
+        const size_t wanted = (size_t)std::min<int64_t>(8, (blocks + num_sms - 1) / num_sms);
+        const size_t resident = std::max<size_t>(1, std::min(wanted, sm / (bytes(K, 1) + own)));
         int kb = KB < K ? KB : K;
-        while (kb > 1 && bytes(K, kb) > kLabelSmemCap) --kb;
+        while (kb > 1 && (bytes(K, kb) > kLabelSmemCap || (bytes(K, kb) + own) * resident > sm)) --kb;
         return kb;
     }
 };
@@ -264,8 +298,10 @@ __device__ __forceinline__ void gauss_labels_tile(const float* __restrict__ x, i
     if (valid) labels[pt] = draw_from_r<P>(sr, t, K, final_, rng, pt);
 }
 
+// At E = 32 and 64 the second launch bound lets the compiler take the registers it needs to load factors ahead (66 ->
+// 126 and 96 -> 136; N = 1.2e5, K = 120: 1440 -> 1100 and 5050 -> 4120 us); at the other widths it costs blocks.
 template <int DP, int P, int E>
-__global__ void __launch_bounds__(P) k_gauss_labels_simt(
+__global__ void __launch_bounds__(P, E == 32 || E == 64 ? 1 : 0) k_gauss_labels_simt(
     const float* __restrict__ x, int64_t N, const float* __restrict__ Wt, const float* __restrict__ bvec,
     const float* __restrict__ cvec, int K, int final_, RngArgs rng, int32_t* __restrict__ labels,
     float* __restrict__ r_out, int kb)
@@ -296,10 +332,10 @@ size_t gauss_label_smem_bytes(int DP, int P, int K)
 
 template <int DP, int P>
 static dpmm_status launch_labels_batched_t(const LabelJob* d_jobs, const int2* d_items, int nitems, int kmax,
-                                           cudaStream_t st)
+                                           int num_sms, cudaStream_t st)
 {
     if (gauss_label_smem_bytes(DP, P, kmax) > kLabelSmemCap) return fail(DPMM_ERR_INVALID_ARG, "too many clusters for the batched label kernel");
-    const int kb = LabelTile<DP, P>::staged(kmax);
+    const int kb = LabelTile<DP, P>::staged(kmax, nitems, num_sms);
     const size_t sm = LabelTile<DP, P>::bytes(kmax, kb);
     auto kern = k_gauss_labels_batched<DP, P>;
     DPMM_TRY(allow_smem(kern, sm, kLabelSmemCap));
@@ -310,25 +346,25 @@ static dpmm_status launch_labels_batched_t(const LabelJob* d_jobs, const int2* d
 
 template <int DP>
 static dpmm_status launch_labels_batched_dp(int P, const LabelJob* d_jobs, const int2* d_items, int nitems, int kmax,
-                                            cudaStream_t st)
+                                            int num_sms, cudaStream_t st)
 {
     switch (P) {
-        case 32: return launch_labels_batched_t<DP, 32>(d_jobs, d_items, nitems, kmax, st);
-        case 64: return launch_labels_batched_t<DP, 64>(d_jobs, d_items, nitems, kmax, st);
-        default: return launch_labels_batched_t<DP, 128>(d_jobs, d_items, nitems, kmax, st);
+        case 32: return launch_labels_batched_t<DP, 32>(d_jobs, d_items, nitems, kmax, num_sms, st);
+        case 64: return launch_labels_batched_t<DP, 64>(d_jobs, d_items, nitems, kmax, num_sms, st);
+        default: return launch_labels_batched_t<DP, 128>(d_jobs, d_items, nitems, kmax, num_sms, st);
     }
 }
 
 dpmm_status launch_labels_batched(int Dp, int P, const LabelJob* d_jobs, const int2* d_items, int nitems, int kmax,
-                                  cudaStream_t st)
+                                  int num_sms, cudaStream_t st)
 {
     switch (Dp) {
-        case 4: return launch_labels_batched_dp<4>(P, d_jobs, d_items, nitems, kmax, st);
-        case 8: return launch_labels_batched_dp<8>(P, d_jobs, d_items, nitems, kmax, st);
-        case 16: return launch_labels_batched_dp<16>(P, d_jobs, d_items, nitems, kmax, st);
-        case 32: return launch_labels_batched_dp<32>(P, d_jobs, d_items, nitems, kmax, st);
-        case 64: return launch_labels_batched_dp<64>(P, d_jobs, d_items, nitems, kmax, st);
-        case 128: return launch_labels_batched_dp<128>(P, d_jobs, d_items, nitems, kmax, st);
+        case 4: return launch_labels_batched_dp<4>(P, d_jobs, d_items, nitems, kmax, num_sms, st);
+        case 8: return launch_labels_batched_dp<8>(P, d_jobs, d_items, nitems, kmax, num_sms, st);
+        case 16: return launch_labels_batched_dp<16>(P, d_jobs, d_items, nitems, kmax, num_sms, st);
+        case 32: return launch_labels_batched_dp<32>(P, d_jobs, d_items, nitems, kmax, num_sms, st);
+        case 64: return launch_labels_batched_dp<64>(P, d_jobs, d_items, nitems, kmax, num_sms, st);
+        case 128: return launch_labels_batched_dp<128>(P, d_jobs, d_items, nitems, kmax, num_sms, st);
         default: return fail(DPMM_ERR_INVALID_ARG, "unsupported padded dimension");
     }
 }
@@ -401,7 +437,7 @@ __global__ void __launch_bounds__(256) k_mult_labels_simt(
 template <int DP, int P, int E>
 static dpmm_status launch_gauss_labels_e(dpmm_ctx* c, int K, int final_, RngArgs r, float* d_rout)
 {
-    const int kb = LabelTile<E, P>::staged(K);
+    const int kb = LabelTile<E, P>::staged(K, blocks_for(c->N, P), c->num_sms);
     const size_t sm = LabelTile<E, P>::bytes(K, kb);
     auto kern = k_gauss_labels_simt<DP, P, E>;
     DPMM_TRY(allow_smem(kern, sm, kLabelSmemCap));

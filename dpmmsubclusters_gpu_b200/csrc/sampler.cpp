@@ -1543,6 +1543,7 @@ static dpmm_status batch_labels(dpmm_batch& b, dpmm_batch::Group& g, const std::
         DPMM_TRY(make_label_job(sm.context(), sm.num_clusters(), st[mem[j]].final_ ? 1 : 0, &g.h_jobs[j]));
     }
     const size_t jb = sizeof(LabelJob) * mem.size();
+    const int num_sms = b.s[mem[0]]->sampler->context()->num_sms;
     int kmax = 1;
     for (size_t j = 0; j < mem.size(); ++j) kmax = std::max(kmax, g.h_jobs[j].K);
     if (g.P == 0 || kmax >= 2 * g.tuned_K) {
@@ -1566,7 +1567,7 @@ static dpmm_status batch_labels(dpmm_batch& b, dpmm_batch::Group& g, const std::
         for (int q = 0; q < 3; ++q) {
             DPMM_TRY(batch_items(b, g, mem, kBatchP[q]));
             DPMM_CUDA_TRY(cudaEventRecord(e0, g.st));
-            DPMM_TRY(launch_labels_batched(g.Dp, kBatchP[q], g.d_jobs, g.d_items, g.nitems, g.kcap, g.st));
+            DPMM_TRY(launch_labels_batched(g.Dp, kBatchP[q], g.d_jobs, g.d_items, g.nitems, g.kcap, num_sms, g.st));
             DPMM_CUDA_TRY(cudaEventRecord(e1, g.st));
             DPMM_CUDA_TRY(cudaEventSynchronize(e1));
             DPMM_CUDA_TRY(cudaEventElapsedTime(&g.tune_ms[q], e0, e1));
@@ -1584,7 +1585,7 @@ static dpmm_status batch_labels(dpmm_batch& b, dpmm_batch::Group& g, const std::
         DPMM_TRY(batch_items(b, g, mem, g.P));
         if (stateful) {
             DPMM_CUDA_TRY(cudaMemcpyAsync(g.d_jobs, g.h_jobs, jb, cudaMemcpyHostToDevice, g.st));
-            DPMM_TRY(launch_labels_batched(g.Dp, g.P, g.d_jobs, g.d_items, g.nitems, g.kcap, g.st));
+            DPMM_TRY(launch_labels_batched(g.Dp, g.P, g.d_jobs, g.d_items, g.nitems, g.kcap, num_sms, g.st));
             ++b.batched_launches;
         }
         return DPMM_OK;
@@ -1599,7 +1600,7 @@ static dpmm_status batch_labels(dpmm_batch& b, dpmm_batch::Group& g, const std::
         cudaGraph_t graph;
         DPMM_CUDA_TRY(cudaStreamBeginCapture(g.st, cudaStreamCaptureModeRelaxed));
         cudaMemcpyAsync(g.d_jobs, g.h_jobs, jb, cudaMemcpyHostToDevice, g.st);
-        dpmm_status ls = launch_labels_batched(g.Dp, g.P, g.d_jobs, g.d_items, g.nitems, g.kcap, g.st);
+        dpmm_status ls = launch_labels_batched(g.Dp, g.P, g.d_jobs, g.d_items, g.nitems, g.kcap, num_sms, g.st);
         cudaError_t ce = cudaStreamEndCapture(g.st, &graph);
         DPMM_TRY(ls);
         DPMM_CUDA_TRY(ce);
