@@ -95,9 +95,10 @@ __device__ double chi2_draw(double k, uint64_t seed, uint64_t draw, uint32_t s, 
 // Bound: three chains one after the other, the factorisation (see BlockChol), the rows of the inverse (8 clocks
 // a term, 2016 terms at D = 64; A^T y = z runs beside it) and the products W = L^-T A.  The variates come from
 // the warps that do not factor, beside the factorisation.  Measured: 300 slots at D = 64 258 -> 85 us, 192 at
-// D = 50 186 -> 67 us, 60 at D = 32 85 -> 40 us.
+// D = 50 186 -> 67 us, 60 at D = 32 85 -> 40 us.  Up to DP = 16 the registers are held to seven blocks an SM: with
+// six, 900 slots at D = 8 need a second wave (31 against 20 us).
 template <int DP>
-__global__ void __launch_bounds__(BlockChol<DP>::T) k_draw_niw(const double* __restrict__ stats, int stat_len, int D,
+__global__ void __launch_bounds__(BlockChol<DP>::T, DP <= 16 ? 7 : 0) k_draw_niw(const double* __restrict__ stats, int stat_len, int D,
                                                               int Dp, double k0, double v0, double ld0,
                                                               const double* __restrict__ prior, double k1, double v1,
                                                               double ld1, const double* __restrict__ prior1,
