@@ -29,9 +29,11 @@ constexpr int kMultChunkUnit = 128;
 // Pruned label phase: at most kMaxKForPrune clusters; a chunk keeps at most kPrMaxCand other
 // clusters before it is evaluated against every cluster.
 constexpr int kMaxKForPrune = 256;
-// Pruned label phase against the tensor-core dense phase (N = 1e7, D = 64 on the B200): the scan alone
-// costs about as much as the dense phase at 7 clusters, and a kept cluster per point about as much as
-// 30 clusters of the dense phase.
+// Pruned label phase against the tensor-core dense phase.  Both constants are those of D = 64: per 1e6 points the
+// pruned phase without kept clusters takes 183 us at K = 8 where the dense one takes 220, and a kept cluster per
+// point takes 590 us where the dense phase takes 19 a cluster.  Dp = 32 uses them too, although its dense kernel
+// works on half the width: 153 against 120 us at K = 8 (157 against 176 at 12), and 150 us a kept cluster against 12 a cluster, so
+// that its own limit would lie near K / 13.
 constexpr int kMinKForPruneTc = 8;
 constexpr double kPruneTcRatio = 30.0;
 constexpr int kPrMaxCand = 16;

@@ -936,10 +936,9 @@ static dpmm_status launch_pruned_dp(dpmm_ctx* c, int K, int final_, const float*
     c->prune_last_extra = extra;
     c->prune_last_over = (int64_t)h[1];
     // each kept cluster costs about one more exact r per point (FP32, in k_prune_draw).  Against the
-    // SIMT dense phase that is the cheaper path up to about 2 per point; the tensor-core dense phase
-    // costs about 1/30 of a kept cluster per point and cluster (N = 1e7, D = 64 on the B200: 0.21 ms
-    // per cluster against 3-6 ms per kept cluster per point), so there the limit is K / 30.  Beyond
-    // it run the dense phase, and wait before the next attempt
+    // SIMT dense phase that is the cheaper path up to about 2 per point; the tensor-core dense phase costs
+    // about 1/30 of a kept cluster per point and cluster at D = 64 (kPruneTcRatio), so there the limit is K / 30.
+    // Beyond it run the dense phase, and wait before the next attempt
     const double limit = tc_dense ? (double)K / kPruneTcRatio : 2.0;
     if (extra > limit || *outside != 0) {
         c->prune_wait = 2;

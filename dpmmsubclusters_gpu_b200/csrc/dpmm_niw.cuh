@@ -85,7 +85,7 @@ static __device__ double mult_lml_block(int D, double n, const double* sum, cons
 // D = 64) and is then factored with shuffles only (14.4e3).  Every element sees the same operations in the
 // same order as in the right-looking form: the results are equal bit for bit.  The other warps compute the
 // terms that need no factor meanwhile.
-// Measured, D = 64: a list of 16 pairs 85 -> 27 us, 300 slots 98 -> 29 us; 2016 pairs at D = 50 263 -> 90 us.
+// Measured, D = 64: a list of 16 pairs 85 -> 27 us, 300 slots 98 -> 29 us; 2016 pairs at D = 50 261 -> 95 us.
 template <int DP>
 struct BlockChol {
     static constexpr int T = DP > 64 ? 256 : 128;                   // threads per block
